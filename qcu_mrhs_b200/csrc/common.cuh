@@ -213,6 +213,10 @@ int sm_count();
 // Resident blocks per SM of `kernel` at `block` threads (cached per kernel and size).
 int blocks_per_sm(const void* kernel, int block, size_t smem = 0);
 
+// Allow `kernel` more than the default 48 KB of shared memory (static and dynamic together):
+// once per kernel, device and larger size.
+int smem_optin(const void* kernel, size_t smem);
+
 // Grid for a grid-stride kernel: enough blocks for the work, at most one full wave.
 template <typename K>
 static int resident_grid(K kernel, int block, int64_t work_items, size_t smem = 0) {

@@ -1,11 +1,12 @@
 // precond.cu -- kernels and host code of the learned gauge-covariant preconditioner
-// (precond.h): the parallel-transport convolution layer, its adjoint (the same kernel
-// with conjugate-transposed spin weights and reversed hops, since T_{+mu}^dag = T_{-mu}),
-// the weight gradient, Adam, the training loss ||M P b - b||^2 / ||b||^2, and the FP64
+// (precond.h): Adam (the parallel-transport layers, their adjoints -- conjugate-transposed
+// spin weights and reversed hops, since T_{+mu}^dag = T_{-mu} -- and the weight gradient are
+// in precond_mma.cu), the training loss ||M P b - b||^2 / ||b||^2, and the FP64
 // kernels of the right-preconditioned BiCGStab.
 //
 // No reference code: the preconditioner is new in this library.  Its CPU restatement
 // (oracle_ptc_forward / _adjoint / _wgrad) is the checker of these kernels.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -21,219 +22,6 @@ int sm_count();
 namespace {
 
 constexpr int kPaths = 9;
-constexpr int kPtcThreads = 256;
-
-__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {   // c + a b
-    c.x = fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x));
-    c.y = fmaf(a.x, b.y, fmaf(a.y, b.x, c.y));
-    return c;
-}
-
-// Path k of full-lattice site `site` (= parity * vh + half index): source site and link
-// (index into the [4][2][Vh] link array; forward links are used as is, backward links
-// conjugate-transposed), and the t-boundary factor.
-__device__ __forceinline__ void ptc_path(const Geom& g, int64_t site, int k, float t_sign, int64_t* src,
-                                         int64_t* link, bool* fwd, float* sg) {
-    const int64_t vh = g.vh;
-    const int p = site >= vh ? 1 : 0;
-    const int64_t idx = site - p * vh;
-    *sg = 1.f;
-    *fwd = true;
-    *link = 0;
-    if (k == 0) {
-        *src = site;
-        return;
-    }
-    const int mu = (k - 1) >> 1;
-    const bool f = ((k - 1) & 1) == 0;
-    const SiteXYZT c = site_coords(g, (uint32_t)idx);
-    const int lxh = g.lxh, Ly = g.L[1], Lz = g.L[2], Lt = g.L[3];
-    const int64_t sy = lxh, sz = (int64_t)lxh * Ly, st = sz * Lz;
-    int64_t nb;
-    bool wrap = false;
-    if (mu == 0) {
-        const int xodd = (p ^ (c.y + c.z + c.t)) & 1;
-        nb = f ? idx - c.xh + (xodd ? (c.xh + 1 == lxh ? 0 : c.xh + 1) : c.xh)
-               : idx - c.xh + (xodd ? c.xh : (c.xh == 0 ? lxh - 1 : c.xh - 1));
-    } else if (mu == 1) {
-        nb = f ? idx + (c.y + 1 == Ly ? -(int64_t)(Ly - 1) * sy : sy) : idx + (c.y == 0 ? (int64_t)(Ly - 1) * sy : -sy);
-    } else if (mu == 2) {
-        nb = f ? idx + (c.z + 1 == Lz ? -(int64_t)(Lz - 1) * sz : sz) : idx + (c.z == 0 ? (int64_t)(Lz - 1) * sz : -sz);
-    } else {
-        wrap = f ? (c.t + 1 == Lt) : (c.t == 0);
-        nb = f ? idx + (wrap ? -(int64_t)(Lt - 1) * st : st) : idx + (wrap ? (int64_t)(Lt - 1) * st : -st);
-    }
-    *src = (int64_t)(1 - p) * vh + nb;
-    *link = f ? ((int64_t)(mu * 2 + p) * vh + idx) : ((int64_t)(mu * 2 + (1 - p)) * vh + nb);
-    *fwd = f;
-    *sg = wrap ? t_sign : 1.f;
-}
-
-// tv = (T_k f)(site) for RHS r: f points at the channel's field + r
-template <int NC>
-__device__ __forceinline__ void ptc_transport(float2 (&tv)[4][NC], const float2* __restrict__ f,
-                                              const float2* __restrict__ gauge, const Geom& g, int64_t site,
-                                              int k, float t_sign, int m) {
-    const int64_t slen = 4 * NC * (int64_t)m;
-    int64_t src, link;
-    bool fwd;
-    float sg;
-    ptc_path(g, site, k, t_sign, &src, &link, &fwd, &sg);
-    const float2* v = f + src * slen;
-    if (k == 0) {
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) tv[s][c] = v[(s * NC + c) * m];
-        return;
-    }
-    const float2* U = gauge + link * (NC * NC);
-    float2 u[NC][NC];
-#pragma unroll
-    for (int a = 0; a < NC; ++a)
-#pragma unroll
-        for (int b = 0; b < NC; ++b) {
-            const float2 e = fwd ? U[a * NC + b] : U[b * NC + a];
-            u[a][b] = make_float2(sg * e.x, fwd ? sg * e.y : -sg * e.y);
-        }
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        float2 in[NC];
-#pragma unroll
-        for (int b = 0; b < NC; ++b) in[b] = v[(s * NC + b) * m];
-#pragma unroll
-        for (int a = 0; a < NC; ++a) {
-            float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int b = 0; b < NC; ++b) acc = cfma(u[a][b], in[b], acc);
-            tv[s][a] = acc;
-        }
-    }
-}
-
-// One layer: out_o = sum_i sum_k W[o][i][k] T_k in_i.  Thread per (site, o, r); the
-// layer's weights are staged in shared memory.
-template <int NC>
-__global__ void __launch_bounds__(kPtcThreads)
-ptc_layer_kernel(float2* __restrict__ out, const float2* __restrict__ in, const float2* __restrict__ w,
-                 const float2* __restrict__ gauge, Geom g, int m, int cin, int cout, float t_sign,
-                 const int* __restrict__ done) {
-    if (done != nullptr && *done) return;
-    extern __shared__ float2 sw[];
-    const int nw = cout * cin * kPaths * 16;
-    for (int e = threadIdx.x; e < nw; e += blockDim.x) sw[e] = w[e];
-    __syncthreads();
-    const int per = m * cout;
-    const int spb = blockDim.x / per;
-    if ((int)threadIdx.x >= spb * per) return;
-    const int r = threadIdx.x % m;
-    const int o = (threadIdx.x / m) % cout;
-    const int64_t slen = 4 * NC * (int64_t)m;
-    const int64_t field = 2 * g.vh * slen;
-    for (int64_t site = (int64_t)blockIdx.x * spb + threadIdx.x / per; site < 2 * g.vh;
-         site += (int64_t)gridDim.x * spb) {
-        float2 acc[4][NC];
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) acc[s][c] = make_float2(0.f, 0.f);
-        for (int k = 0; k < kPaths; ++k) {
-            for (int i = 0; i < cin; ++i) {
-                float2 tv[4][NC];
-                ptc_transport<NC>(tv, in + i * field + r, gauge, g, site, k, t_sign, m);
-                const float2* W = sw + ((o * cin + i) * kPaths + k) * 16;
-#pragma unroll
-                for (int sp = 0; sp < 4; ++sp)
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) {
-                        const float2 wv = W[sp * 4 + s];
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) acc[sp][c] = cfma(wv, tv[s][c], acc[sp][c]);
-                    }
-            }
-        }
-        float2* dst = out + o * field + site * slen + r;
-#pragma unroll
-        for (int s = 0; s < 4; ++s)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) dst[(s * NC + c) * m] = acc[s][c];
-    }
-}
-
-// gw[o][i][k][s'][s] = sum_{site, c, r} gout_o[s'][c][r] conj((T_k in_i)[s][c][r]); one block
-// per (o, i, k), fixed thread-to-element assignment and a fixed reduction order.
-template <int NC>
-__global__ void __launch_bounds__(kPtcThreads)
-ptc_wgrad_kernel(double2* __restrict__ gw, const float2* __restrict__ gout, const float2* __restrict__ in,
-                 const float2* __restrict__ gauge, Geom g, int m, int cin, int cout, float t_sign) {
-    const int q = blockIdx.x;
-    const int k = q % kPaths, i = (q / kPaths) % cin, o = q / (kPaths * cin);
-    const int spb = kPtcThreads / m;
-    const int r = threadIdx.x % m;
-    const int64_t slen = 4 * NC * (int64_t)m;
-    const int64_t field = 2 * g.vh * slen;
-    double2 acc[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = make_double2(0.0, 0.0);
-    if ((int)threadIdx.x < spb * m) {
-        for (int64_t site = threadIdx.x / m; site < 2 * g.vh; site += spb) {
-            float2 tv[4][NC], gv[4][NC];
-            ptc_transport<NC>(tv, in + i * field + r, gauge, g, site, k, t_sign, m);
-            const float2* gp = gout + o * field + site * slen + r;
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-#pragma unroll
-                for (int c = 0; c < NC; ++c) gv[s][c] = gp[(s * NC + c) * m];
-#pragma unroll
-            for (int sp = 0; sp < 4; ++sp)
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    float2 a = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c)
-                        a = cfma(gv[sp][c], make_float2(tv[s][c].x, -tv[s][c].y), a);
-                    acc[sp * 4 + s].x += a.x;
-                    acc[sp * 4 + s].y += a.y;
-                }
-        }
-    }
-    __shared__ double2 red[kPtcThreads / 32][16];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-        double x = acc[e].x, y = acc[e].y;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            x += __shfl_down_sync(0xffffffffu, x, off);
-            y += __shfl_down_sync(0xffffffffu, y, off);
-        }
-        if (lane == 0) red[warp][e] = make_double2(x, y);
-    }
-    __syncthreads();
-    if (threadIdx.x < 16) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int wi = 0; wi < kPtcThreads / 32; ++wi) {
-            s.x += red[wi][threadIdx.x].x;
-            s.y += red[wi][threadIdx.x].y;
-        }
-        gw[(int64_t)q * 16 + threadIdx.x] = s;
-    }
-}
-
-__device__ __forceinline__ int opposite_path(int k) { return k == 0 ? 0 : (((k - 1) & 1) ? k - 1 : k + 1); }
-
-// wadj[i][o][-k] = W[o][i][k]^dag (spin conjugate transpose): the adjoint layer
-__global__ void ptc_adjoint_weights_kernel(float2* __restrict__ wadj, const float2* __restrict__ w, int cin,
-                                           int cout) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= cout * cin * kPaths * 16) return;
-    const int s = e & 3, sp = (e >> 2) & 3;
-    const int k = (e >> 4) % kPaths;
-    const int i = (e / (16 * kPaths)) % cin;
-    const int o = e / (16 * kPaths * cin);
-    const float2 v = w[e];
-    wadj[(((int64_t)i * cout + o) * kPaths + opposite_path(k)) * 16 + s * 4 + sp] = make_float2(v.x, -v.y);
-}
 
 // Adam on the real and imaginary parts; the gradient of the real loss with respect to
 // (Re w, Im w) is 2 gw.
@@ -346,61 +134,6 @@ int red_grid(K k, int block, int64_t n, const Scratch& ws) {
     return grid > ws.max_blocks ? ws.max_blocks : grid;
 }
 
-template <int NC>
-int layer_launch(float2* out, const float2* in, const float2* w, const float2* gauge, const Geom& g, int m, int cin,
-                 int cout, float t_sign, const int* done, cudaStream_t st) {
-    const size_t smem = (size_t)cout * cin * kPaths * 16 * sizeof(float2);
-    if (smem > 200 * 1024) return set_error(QCU_ERR_UNSUPPORTED, "layer weights exceed shared memory");
-    const int per = m * cout;
-    const int block = per <= kPtcThreads ? (kPtcThreads / per) * per : per;
-    if (block > 1024) return set_error(QCU_ERR_UNSUPPORTED, "m_rhs * channels = %d > 1024", per);
-    const int spb = block / per;
-    const int64_t want = (2 * g.vh + spb - 1) / spb;
-    const int64_t cap = (int64_t)sm_count() * 8;
-    const int grid = (int)(want < cap ? want : cap);
-    ptc_layer_kernel<NC><<<grid, block, smem, st>>>(out, in, w, gauge, g, m, cin, cout, t_sign, done);
-    QCUB_CHECK_LAUNCH();
-    return QCU_SUCCESS;
-}
-
-template <int NC>
-int wgrad_launch(double2* gw, const float2* gout, const float2* in, const float2* gauge, const Geom& g, int m,
-                 int cin, int cout, float t_sign, cudaStream_t st) {
-    ptc_wgrad_kernel<NC><<<cout * cin * kPaths, kPtcThreads, 0, st>>>(gw, gout, in, gauge, g, m, cin, cout, t_sign);
-    QCUB_CHECK_LAUNCH();
-    return QCU_SUCCESS;
-}
-
-// raise the dynamic shared memory limit of the layer kernels (weights of one layer);
-// done once at set-up, outside any stream capture
-int ptc_set_attributes() {
-    const int bytes = 200 * 1024;
-    QCUB_CUDA_CHECK(cudaFuncSetAttribute(ptc_layer_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    QCUB_CUDA_CHECK(cudaFuncSetAttribute(ptc_layer_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    QCUB_CUDA_CHECK(cudaFuncSetAttribute(ptc_layer_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    return QCU_SUCCESS;
-}
-
-int layer(int nc, float2* out, const float2* in, const float2* w, const float2* gauge, const Geom& g, int m, int cin,
-          int cout, float t_sign, const int* done, cudaStream_t st) {
-    switch (nc) {
-        case 2: return layer_launch<2>(out, in, w, gauge, g, m, cin, cout, t_sign, done, st);
-        case 3: return layer_launch<3>(out, in, w, gauge, g, m, cin, cout, t_sign, done, st);
-        case 4: return layer_launch<4>(out, in, w, gauge, g, m, cin, cout, t_sign, done, st);
-        default: return set_error(QCU_ERR_UNSUPPORTED, "preconditioner n_color=%d (2..4)", nc);
-    }
-}
-
-int wgrad(int nc, double2* gw, const float2* gout, const float2* in, const float2* gauge, const Geom& g, int m,
-          int cin, int cout, float t_sign, cudaStream_t st) {
-    switch (nc) {
-        case 2: return wgrad_launch<2>(gw, gout, in, gauge, g, m, cin, cout, t_sign, st);
-        case 3: return wgrad_launch<3>(gw, gout, in, gauge, g, m, cin, cout, t_sign, st);
-        case 4: return wgrad_launch<4>(gw, gout, in, gauge, g, m, cin, cout, t_sign, st);
-        default: return set_error(QCU_ERR_UNSUPPORTED, "preconditioner n_color=%d (2..4)", nc);
-    }
-}
-
 }  // namespace
 
 // ---------------- FP64 pieces of the preconditioned solve ----------------
@@ -500,9 +233,17 @@ int Precond::init(const int L[4], int n_color, int m_rhs, int n_layers, int chan
         woff.push_back(nw);
         nw += (int64_t)cout[l] * cin[l] * kPaths * 16;
     }
+    size_t fb = 0, fa = 0, gb = 0;
+    for (int l = 0; l < layers; ++l) {
+        foff.push_back(fb);
+        faoff.push_back(fa);
+        fb += ptc_frag_bytes(cin[l], cout[l]);
+        fa += ptc_frag_bytes(cout[l], cin[l]);
+        gb = std::max(gb, ptc_grad_bytes(cin[l], cout[l]));
+    }
     int rc;
-    if ((rc = ptc_set_attributes())) return rc;
-    if ((rc = w.ensure(nw * sizeof(float2))) || (rc = wadj.ensure(nw * sizeof(float2))) ||
+    if ((rc = w.ensure(nw * sizeof(float2))) || (rc = frag.ensure(fb)) || (rc = fragadj.ensure(fa)) ||
+        (rc = gpart.ensure(gb)) ||
         (rc = gw.ensure(nw * sizeof(double2))) || (rc = m1.ensure(nw * sizeof(float2))) ||
         (rc = m2.ensure(nw * sizeof(float2))))
         return rc;
@@ -526,8 +267,19 @@ int Precond::init(const int L[4], int n_color, int m_rhs, int n_layers, int chan
     QCUB_CUDA_CHECK(cudaMemsetAsync(w.ptr, 0, nw * sizeof(float2), stream));
     QCUB_CUDA_CHECK(cudaMemsetAsync(m1.ptr, 0, nw * sizeof(float2), stream));
     QCUB_CUDA_CHECK(cudaMemsetAsync(m2.ptr, 0, nw * sizeof(float2), stream));
+    if ((rc = prepare(false, stream))) return rc;
     QCUB_CUDA_CHECK(cudaStreamSynchronize(stream));
     return QCU_SUCCESS;
+}
+
+int Precond::prepare(bool adj, cudaStream_t st) {
+    const float2* ws_[16];
+    void* fs[16];
+    for (int l = 0; l < layers; ++l) {
+        ws_[l] = static_cast<const float2*>(w.ptr) + woff[l];
+        fs[l] = static_cast<char*>(adj ? fragadj.ptr : frag.ptr) + (adj ? faoff[l] : foff[l]);
+    }
+    return ptc_prepare(ws_, fs, cin.data(), cout.data(), layers, adj, st);
 }
 
 void Precond::release() {
@@ -541,13 +293,13 @@ void Precond::release() {
 
 int Precond::apply(float2* out, const float2* in, const void* gauge32, cudaStream_t st, const int* done) {
     const float2* gp = static_cast<const float2*>(gauge32);
-    const float2* wp = static_cast<const float2*>(w.ptr);
     float2* fields = static_cast<float2*>(act.ptr);
     const int64_t fl = field_len();
     const float2* src = in;
     for (int l = 0; l < layers; ++l) {
         float2* dst = (l == layers - 1) ? out : fields + (int64_t)act_offset(l + 1) * fl;
-        const int rc = layer(nc, dst, src, wp + woff[l], gp, g, m, cin[l], cout[l], (float)t_sign, done, st);
+        const int rc = ptc_layer(nc, dst, src, static_cast<const char*>(frag.ptr) + foff[l], gp, g, m, cin[l], cout[l],
+                                 (float)t_sign, done, st);
         if (rc) return rc;
         src = dst;
     }
@@ -557,7 +309,6 @@ int Precond::apply(float2* out, const float2* in, const void* gauge32, cudaStrea
 int Precond::loss_grad(const float2* b, double kappa, double* loss, cudaStream_t st) {
     if (!has_gauge) return set_error(QCU_ERR_STATE, "preconditioner gauge field not set");
     const float2* gp = static_cast<const float2*>(gauge.ptr);
-    const float2* wp = static_cast<const float2*>(w.ptr);
     float2* fields = static_cast<float2*>(act.ptr);
     const int64_t fl = field_len();
     const int64_t len = fl / m;   // complex per RHS
@@ -565,8 +316,9 @@ int Precond::loss_grad(const float2* b, double kappa, double* loss, cudaStream_t
     // forward, keeping every layer's input
     QCUB_CUDA_CHECK(cudaMemcpyAsync(fields, b, field_bytes(), cudaMemcpyDeviceToDevice, st));
     for (int l = 0; l < layers; ++l) {
-        if ((rc = layer(nc, fields + (int64_t)act_offset(l + 1) * fl, fields + (int64_t)act_offset(l) * fl,
-                        wp + woff[l], gp, g, m, cin[l], cout[l], (float)t_sign, nullptr, st)))
+        if ((rc = ptc_layer(nc, fields + (int64_t)act_offset(l + 1) * fl, fields + (int64_t)act_offset(l) * fl,
+                            static_cast<const char*>(frag.ptr) + foff[l], gp, g, m, cin[l], cout[l], (float)t_sign,
+                            nullptr, st)))
             return rc;
     }
     const float2* y = fields + (int64_t)act_offset(layers) * fl;
@@ -583,19 +335,17 @@ int Precond::loss_grad(const float2* b, double kappa, double* loss, cudaStream_t
     scale_rhs_kernel<<<elem_grid(fl), 256, 0, st>>>(seed, dn + kMaxRhs, fl, m);
     QCUB_CHECK_LAUNCH();
     // backward
+    if ((rc = prepare(true, st))) return rc;
     int cur = 0;
     for (int l = layers - 1; l >= 0; --l) {
         const float2* gout = static_cast<const float2*>(gbuf[cur].ptr);
-        if ((rc = wgrad(nc, static_cast<double2*>(gw.ptr) + woff[l], gout, fields + (int64_t)act_offset(l) * fl, gp, g,
-                        m, cin[l], cout[l], (float)t_sign, st)))
+        if ((rc = ptc_grad(nc, static_cast<double2*>(gw.ptr) + woff[l], gpart.ptr, gout,
+                           fields + (int64_t)act_offset(l) * fl, gp, g, m, cin[l], cout[l], (float)t_sign, st)))
             return rc;
         if (l == 0) break;
-        const int nwl = cout[l] * cin[l] * kPaths * 16;
-        float2* wa = static_cast<float2*>(wadj.ptr) + woff[l];
-        ptc_adjoint_weights_kernel<<<(nwl + 255) / 256, 256, 0, st>>>(wa, wp + woff[l], cin[l], cout[l]);
-        QCUB_CHECK_LAUNCH();
-        if ((rc = layer(nc, static_cast<float2*>(gbuf[1 - cur].ptr), gout, wa, gp, g, m, cout[l], cin[l],
-                        (float)t_sign, nullptr, st)))
+        if ((rc = ptc_layer(nc, static_cast<float2*>(gbuf[1 - cur].ptr), gout,
+                            static_cast<const char*>(fragadj.ptr) + faoff[l], gp, g, m, cout[l], cin[l], (float)t_sign,
+                            nullptr, st)))
             return rc;
         cur = 1 - cur;
     }
@@ -619,7 +369,7 @@ int Precond::adam(double lr, cudaStream_t st) {
                                                          static_cast<const double2*>(gw.ptr), nw, (float)lr, b1, b2,
                                                          1e-8f, c1, c2);
     QCUB_CHECK_LAUNCH();
-    return QCU_SUCCESS;
+    return prepare(false, st);
 }
 
 }  // namespace qcub
@@ -680,6 +430,7 @@ int qcuPrecondSetWeights(void* handle, const float* weights) {
     QCUB_CUDA_CHECK(cudaMemcpyAsync(P.w.ptr, weights, P.nw * sizeof(float2), cudaMemcpyHostToDevice, P.stream));
     QCUB_CUDA_CHECK(cudaMemsetAsync(P.m1.ptr, 0, P.nw * sizeof(float2), P.stream));
     QCUB_CUDA_CHECK(cudaMemsetAsync(P.m2.ptr, 0, P.nw * sizeof(float2), P.stream));
+    if (int rc = P.prepare(false, P.stream)) return rc;
     QCUB_CUDA_CHECK(cudaStreamSynchronize(P.stream));
     P.step = 0;
     return QCU_SUCCESS;

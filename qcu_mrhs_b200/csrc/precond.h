@@ -22,11 +22,14 @@ struct Precond {
     std::vector<int> cin, cout;
     std::vector<int64_t> woff;      // complex offset of each layer's weights
     int64_t nw = 0;                 // complex weights in total
-    DevBuf w, wadj, gw, m1, m2;     // weights, adjoint weights, gradient (double2), Adam moments
+    DevBuf w, gw, m1, m2;           // weights, gradient (double2), Adam moments
+    DevBuf frag, fragadj;           // MMA fragments of the weights, of the layers and the adjoint layers
+    std::vector<size_t> foff, faoff;   // byte offset of each layer's fragments
     DevBuf gauge;                   // FP32 gauge of the training API
     bool has_gauge = false;
     DevBuf act;                     // layer inputs/outputs: 1 + C (layers - 1) + 1 fields
     DevBuf gbuf[2];                 // gradient ping-pong, C fields each
+    DevBuf gpart;                   // partial sums of one layer's weight gradient
     DevBuf tmp[3];                  // loss temporaries (one field each)
     DevBuf norms;                   // device double[2 * kMaxRhs]
     double* host_norms = nullptr;   // pinned mirror
@@ -40,12 +43,31 @@ struct Precond {
 
     int init(const int L[4], int n_color, int m_rhs, int n_layers, int channels, double t_boundary);
     void release();
+    // MMA fragments of the current weights (adj: of the adjoint layers)
+    int prepare(bool adj, cudaStream_t st);
     // out = P in (FP32 fields); gauge: FP32 EO gauge; kernels return at once once *done is set
     int apply(float2* out, const float2* in, const void* gauge32, cudaStream_t st, const int* done = nullptr);
     // loss = sum_j ||M P b_j - b_j||^2 / ||b_j||^2 and the weight gradient into gw
     int loss_grad(const float2* b, double kappa, double* loss, cudaStream_t st);
     int adam(double lr, cudaStream_t st);
 };
+
+// ---- layers (precond_mma.cu) ----
+// bytes of one layer's weight fragments
+size_t ptc_frag_bytes(int cin, int cout);
+// fragments of `layers` (<= 16) layers from their weights [cout][cin][9][4][4]; adj: of the
+// adjoint layers, from the same weights
+int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
+                cudaStream_t st);
+// out_o = sum_i sum_k W[o][i][k] T_k in_i
+int ptc_layer(int nc, float2* out, const float2* in, const void* frag, const float2* gauge, const Geom& g, int m,
+              int cin, int cout, float t_sign, const int* done, cudaStream_t st);
+
+// weight gradient gw[o][i][k][s'][s] = sum gout_o[s'] conj((T_k in_i)[s]); part: scratch of
+// ptc_grad_bytes
+size_t ptc_grad_bytes(int cin, int cout);
+int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge, const Geom& g,
+             int m, int cin, int cout, float t_sign, cudaStream_t st);
 
 // Right-preconditioned BiCGStab on the full system M x = b (solver.cu).
 int solve_precond(Context& c, Precond* P, void* x, const void* b, int max_iter, double tol);

@@ -1,0 +1,784 @@
+// precond_mma.cu -- tensor-core kernels of the learned preconditioner (precond.h).
+//
+// Layer: out_o(x) = sum_k U_k(x) [ sum_i W[o][i][k] in_i(x + k) ], k = 0..8, with U_0 = 1.
+// The spin mixing in brackets is one matrix product per path, the same weights for every
+// column (site, colour, RHS): A (rows (o, s', re/im), K = (i, s, re/im)) times B (the raw
+// neighbour spinors).  The link acts on the product's colours, in FP32.
+//
+// FP32 products on the 16-bit MMA (mma.sync m16n8k16, FP32 accumulation): operands are scaled
+// by powers of two so that their largest entries sit at 2^14 (the weights per layer, every
+// column of a field per path), split into FP16 pieces, and the pieces' products accumulated.
+//   first piece  the value rounded to a multiple of 2^6, so 9 bits of the largest entry.  Products
+//                of two first pieces are multiples of 2^12 below 2^30, and 64 of them (the K of a
+//                path) add up within 24 bits: exact.
+//   the rest     weights w = w0 + w1 + w2 (w1, w2 of 11 bits each: all 24 bits), fields
+//                x = x0 + x1 (x1 = fp16(x - x0), an error of random sign below 2^-22 of the largest
+//                entry); w0 x1 + w1 x0 + w2 x0 + w1 x1.
+// The exactness of the first product matters because the MMA truncates: it keeps 2 bits
+// below FP32's last place of the largest addend and rounds the sum toward zero (measured: with
+// 11-bit pieces a sum over K = 64 is short by 9e-8 of itself on average).  That bias and what is
+// lost of the weights are the same at every site, so they add up in the weight gradient:
+// 1.1e-6 of it, against 3.5e-8 with FP32 arithmetic.  One path's product is accumulated from
+// zero and added to the FP32 result outside the MMA, so the sums are chains of at most 9 FP32
+// additions.
+//
+// Fragments (PTX ISA, mma.m16n8k16): lane 4 g + t holds A rows g, g + 8 at K 2t..2t+1 and
+// 2t+8..2t+9, B column g at the same K, D rows g, g + 8 at columns 2t, 2t + 1.  K-step j holds
+// channels 2j (K 0..7) and 2j + 1 (K 8..15), each as 4 spins (re, im): lane t loads spin t of
+// column g.  Rows 0..7 of a tile are the real parts of two output channels x 4 spins, rows
+// 8..15 the imaginary parts: a lane's D registers are whole complex numbers.
+//
+// No reference code; the CPU restatement oracle_ptc_forward is the checker.
+#include "precond.h"
+
+namespace qcub {
+
+int sm_count();
+
+namespace {
+
+constexpr int kPaths = 9;
+constexpr int kMmaThreads = 256;
+constexpr int kPieces = 3;                        // of a weight
+constexpr int kStepVecs = kPieces * 32;           // uint4 of one (path, row tile, K step)
+constexpr int kStepBytes = kStepVecs * 16;
+
+__device__ __forceinline__ void mma16(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+
+// the same from a zero accumulator
+__device__ __forceinline__ void mma16_zero(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+__device__ __forceinline__ uint32_t half_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+
+// v (below 2^15) rounded to a multiple of 2^(15 - BITS): adding 1.5 x 2^(38 - BITS) leaves no
+// lower bits
+template <int BITS>
+__device__ __forceinline__ float round_first(float v) {
+    constexpr float c = 1.5f * (float)(1ull << (38 - BITS));
+    return __fadd_rn(__fadd_rn(v, c), -c);
+}
+// first (BITS bits) and second FP16 pair of the pair v (scaled)
+template <int BITS>
+__device__ __forceinline__ void split16(float2 v, uint32_t& hi, uint32_t& lo) {
+    const float2 f = make_float2(round_first<BITS>(v.x), round_first<BITS>(v.y));
+    hi = half_bits(__float22half2_rn(f));   // exact
+    lo = half_bits(__floats2half2_rn(v.x - f.x, v.y - f.y));
+}
+// three FP16 pairs
+__device__ __forceinline__ void split16x3(float2 v, uint32_t& h0, uint32_t& h1, uint32_t& h2) {
+    const float2 f = make_float2(round_first<9>(v.x), round_first<9>(v.y)), r = make_float2(v.x - f.x, v.y - f.y);
+    const __half2 b = __float22half2_rn(r);
+    const float2 e = __half22float2(b);
+    h0 = half_bits(__float22half2_rn(f));
+    h1 = half_bits(b);
+    h2 = half_bits(__floats2half2_rn(r.x - e.x, r.y - e.y));
+}
+
+// power of two that brings a maximum m into [2^14, 2^15), and its inverse
+__device__ __forceinline__ float scale_to_half(float m, float* inv) {
+    const int eb = (int)((__float_as_uint(m) >> 23) & 255u);
+    const int f = min(max(268 - eb, 1), 253);
+    *inv = __uint_as_float((uint32_t)(254 - f) << 23);
+    return __uint_as_float((uint32_t)f << 23);
+}
+
+// ---- weights ----
+// A fragments of one layer: [path][row tile][K step][piece][lane] uint4, then at the end the
+// inverse of the layer's scale.  adj: of the adjoint layer, W'[i][o][-k] = W[o][i][k]^dag.
+struct FragShape {
+    int mt, ks;        // row tiles (2 output channels each) and K steps (2 input channels), padded
+    int tiles, steps;  // per block and per channel chunk
+};
+
+FragShape frag_shape(int cin, int cout) {
+    FragShape s;
+    s.steps = cin <= 2 ? 1 : (cin <= 4 ? 2 : (cin <= 8 ? 4 : 2));
+    s.ks = (cin + 2 * s.steps - 1) / (2 * s.steps) * s.steps;
+    s.tiles = cout <= 2 ? 1 : (cout <= 4 ? 2 : 4);
+    if (s.tiles == 4 && (size_t)kPaths * 4 * s.ks * kStepBytes > 224 * 1024) s.tiles = 2;
+    s.mt = (cout + 2 * s.tiles - 1) / (2 * s.tiles) * s.tiles;
+    return s;
+}
+
+struct PrepLayer {
+    const float2* w;
+    uint4* frag;
+    float* inv;
+    int cin, cout;     // of the layer that the fragments compute
+    int mt, ks;
+};
+struct PrepArgs {
+    PrepLayer l[16];
+    int adj;
+};
+
+__device__ __forceinline__ int opposite_path(int k) { return k == 0 ? 0 : (((k - 1) & 1) ? k - 1 : k + 1); }
+
+__global__ void ptc_prepare_kernel(PrepArgs a) {
+    const PrepLayer L = a.l[blockIdx.x];
+    const int n = L.cin * L.cout * kPaths * 16;
+    __shared__ float wmax[32];
+    float mx = 0.f;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) mx = fmaxf(mx, fmaxf(fabsf(L.w[e].x), fabsf(L.w[e].y)));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = 0.f;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) mx = fmaxf(mx, wmax[i]);
+    float inv;
+    const float sc = scale_to_half(mx, &inv);
+    if (threadIdx.x == 0) *L.inv = inv;
+    const int total = kPaths * L.mt * L.ks * 32;
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+        const int lane = e & 31, j = (e >> 5) % L.ks, q = (e >> 5) / L.ks;
+        const int mt = q % L.mt, k = q / L.mt;
+        const int g = lane >> 2, t = lane & 3;
+        const int o = 2 * mt + (g >> 2), sp = g & 3;
+        uint32_t w0[4], w1[4], w2[4];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int i = 2 * j + c;
+            float2 v = make_float2(0.f, 0.f);
+            if (o < L.cout && i < L.cin) {
+                if (a.adj) {   // stored W[o' = i][i' = o][opposite k][s' = t][s = sp]
+                    v = L.w[((int64_t)(i * L.cout + o) * kPaths + opposite_path(k)) * 16 + t * 4 + sp];
+                    v.y = -v.y;
+                } else {
+                    v = L.w[((int64_t)(o * L.cin + i) * kPaths + k) * 16 + sp * 4 + t];
+                }
+            }
+            v.x *= sc;
+            v.y *= sc;
+            split16x3(make_float2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
+            split16x3(make_float2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
+        }
+        uint4* f = L.frag + (int64_t)(e >> 5) * kStepVecs + lane;
+        f[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+        f[32] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+        f[64] = make_uint4(w2[0], w2[1], w2[2], w2[3]);
+    }
+}
+
+// ---- layer ----
+struct LayerArgs {
+    float2* out;
+    const float2* in;
+    const uint4* frag;
+    const float* inv;
+    const float2* gauge;
+    Geom g;
+    int m, cin, cout, mt, ks;
+    float t_sign;
+    const int* done;
+};
+
+// full-lattice site (even half first) as coordinates
+struct PtcSite {
+    int p, xh, y, z, t;
+    uint32_t idx;
+};
+__device__ __forceinline__ PtcSite ptc_site(const Geom& g, uint32_t site) {
+    PtcSite s;
+    s.p = site >= (uint32_t)g.vh;
+    s.idx = site - (s.p ? (uint32_t)g.vh : 0u);
+    const SiteXYZT c = site_coords(g, s.idx);
+    s.xh = c.xh;
+    s.y = c.y;
+    s.z = c.z;
+    s.t = c.t;
+    return s;
+}
+// path k >= 1 of a site: source site (full lattice), link (index into [4][2][Vh]; backward links
+// are conjugate-transposed) and whether it crosses the t boundary
+__device__ __forceinline__ void ptc_step(const Geom& g, const PtcSite& s, int k, uint32_t& src, uint32_t& link, bool& wrap) {
+    const uint32_t vh = (uint32_t)g.vh, lxh = (uint32_t)g.lxh, Ly = (uint32_t)g.L[1], Lz = (uint32_t)g.L[2],
+                   Lt = (uint32_t)g.L[3];
+    const uint32_t sy = lxh, sz = lxh * Ly, st = sz * Lz, xh = (uint32_t)s.xh;
+    const int mu = (k - 1) >> 1;
+    const bool f = ((k - 1) & 1) == 0;
+    uint32_t nb;
+    wrap = false;
+    if (mu == 0) {
+        const bool xodd = ((s.p ^ (s.y + s.z + s.t)) & 1) != 0;
+        const uint32_t row = s.idx - xh;
+        nb = row + (f ? (xodd ? (xh + 1 == lxh ? 0u : xh + 1) : xh) : (xodd ? xh : (xh == 0 ? lxh - 1 : xh - 1)));
+    } else if (mu == 1) {
+        nb = f ? s.idx + sy - ((uint32_t)s.y + 1 == Ly ? Ly * sy : 0u) : s.idx - sy + (s.y == 0 ? Ly * sy : 0u);
+    } else if (mu == 2) {
+        nb = f ? s.idx + sz - ((uint32_t)s.z + 1 == Lz ? Lz * sz : 0u) : s.idx - sz + (s.z == 0 ? Lz * sz : 0u);
+    } else {
+        wrap = f ? (uint32_t)s.t + 1 == Lt : s.t == 0;
+        nb = f ? s.idx + st - (wrap ? Lt * st : 0u) : s.idx - st + (wrap ? Lt * st : 0u);
+    }
+    src = (s.p ? 0u : vh) + nb;
+    link = (uint32_t)(2 * mu + (f ? s.p : 1 - s.p)) * vh + (f ? s.idx : nb);
+}
+
+// two FP32 numbers in one register pair and their packed arithmetic (same rounding as the
+// scalar instructions, half the issue slots)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ float2 cfma2(float2 a, float2 b, float2 c) {   // c + a b
+    c.x = fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x));
+    c.y = fmaf(a.x, b.y, fmaf(a.y, b.x, c.y));
+    return c;
+}
+
+// One warp per tile of 8 consecutive columns (site, RHS) of the flattened full lattice, all
+// colours, 2 MT output channels.  The block's weights (its MT row tiles) stay in shared memory
+// (216 KB for 8 x 8 channels), so one block of 8 warps runs on an SM, at 255 registers: a
+// step's spinors and link are requested under the products of the step before it.  16^4,
+// SU(3), m = 8, one 8 -> 8 layer: 7.0 ms as FP32 arithmetic with a thread per (site, output
+// channel, RHS), each transporting every input again; 2.07 ms with 12 warps and no prefetch;
+// 1.85 ms so.  5 MT KS NC = 240 MMAs a path bound it at 1.05 ms; the rest is latency that 8
+// warps do not cover.
+template <int NC, int MT, int KS>
+__global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs a) {
+    if (a.done != nullptr && *a.done) return;
+    extern __shared__ uint4 sw[];
+    const int mt0 = blockIdx.y * MT;
+    const int per_path = MT * a.ks * kStepVecs;
+    for (int e = threadIdx.x; e < kPaths * per_path; e += blockDim.x) {
+        const int k = e / per_path, r = e - k * per_path;
+        sw[e] = a.frag[(int64_t)(k * a.mt + mt0) * a.ks * kStepVecs + r];
+    }
+    __syncthreads();
+    const float winv = *a.inv;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int m = a.m;
+    const uint32_t um = (uint32_t)m;
+    const uint32_t cols = 2u * (uint32_t)a.g.vh * um;
+    const int64_t slen = 4 * NC * (int64_t)m, field = 2 * a.g.vh * slen;
+    const bool odd = (m & 1) != 0;   // the columns 2t, 2t + 1 may belong to two sites
+    const uint32_t nw = gridDim.x * (kMmaThreads / 32);
+    for (uint32_t tile = blockIdx.x * (kMmaThreads / 32) + (threadIdx.x >> 5); tile * 8 < cols; tile += nw) {
+        const uint32_t col = min(tile * 8 + g, cols - 1);
+        const uint32_t site = col / um, r = col - site * um;
+        const PtcSite ps = ptc_site(a.g, site);
+        const float2* const in = a.in + (int64_t)(t * NC) * m + r;
+        // output of this lane's rows, columns (2t, 2t + 1) as pairs
+        f32x2 re[MT][NC], im[MT][NC];
+#pragma unroll
+        for (int q = 0; q < MT; ++q)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) re[q][c] = im[q][c] = 0ull;
+        // a step: path k, channel chunk j0; its spinors (spin t, column g) are requested before the
+        // products of the step before it
+        float2 x[2 * KS][NC];
+        uint32_t link = 0;
+        bool wrap = false;
+        float2 u0[NC][NC];   // link of column 2t, as stored (transposed for backward paths)
+        auto load = [&](int k, int j0) {
+            uint32_t src = site;
+            if (k) {
+                ptc_step(a.g, ps, k, src, link, wrap);
+                const float2* U = a.gauge + (int64_t)__shfl_sync(0xffffffffu, link, 8 * t) * (NC * NC);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int d = 0; d < NC; ++d) u0[c][d] = __ldg(U + ((k & 1) ? c * NC + d : d * NC + c));
+            }
+            const float2* v = in + (int64_t)src * slen;
+#pragma unroll
+            for (int i = 0; i < 2 * KS; ++i) {
+                // channels past the last meet zero weights: any finite number of the field will do
+                const float2* vi = v + (int64_t)min(2 * j0 + i, a.cin - 1) * field;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) x[i][c] = __ldg(vi + c * m);
+            }
+        };
+        load(0, 0);
+#pragma unroll 1
+        for (int k = 0, j0 = 0; k < kPaths;) {
+            float mx = 0.f;
+#pragma unroll
+            for (int i = 0; i < 2 * KS; ++i)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) mx = fmaxf(mx, fmaxf(fabsf(x[i][c].x), fabsf(x[i][c].y)));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            float inv;
+            const float sc = scale_to_half(mx, &inv);
+            uint32_t bh[2 * KS][NC], bl[2 * KS][NC];
+#pragma unroll
+            for (int i = 0; i < 2 * KS; ++i)
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    split16<9>(make_float2(x[i][c].x * sc, x[i][c].y * sc), bh[i][c], bl[i][c]);
+            // scale, link and boundary of this lane's D columns 2t and 2t + 1; the scale goes into
+            // the link
+            float dinv[2];
+            f32x2 ur[NC][NC], ui[NC][NC];
+#pragma unroll
+            for (int b = 0; b < 2; ++b) dinv[b] = __shfl_sync(0xffffffffu, inv, 8 * t + 4 * b);
+            if (k) {
+                const bool fwd = (k & 1) != 0;
+                const int w0 = __shfl_sync(0xffffffffu, (int)wrap, 8 * t), w1 = __shfl_sync(0xffffffffu, (int)wrap, 8 * t + 4);
+                const uint32_t l1 = __shfl_sync(0xffffffffu, link, 8 * t + 4);
+                const float s0 = w0 ? a.t_sign * dinv[0] : dinv[0], s1 = w1 ? a.t_sign * dinv[1] : dinv[1];
+                const float2* U = a.gauge + (int64_t)l1 * (NC * NC);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int d = 0; d < NC; ++d) {
+                        float2 e = u0[c][d];
+                        if (odd) e = __ldg(U + (fwd ? c * NC + d : d * NC + c));
+                        ur[c][d] = pack2(u0[c][d].x * s0, e.x * s1);
+                        ui[c][d] = pack2(u0[c][d].y * (fwd ? s0 : -s0), e.y * (fwd ? s1 : -s1));
+                    }
+            }
+            const int k0 = k, j00 = j0;
+            j0 += KS;
+            if (j0 >= a.ks) {
+                j0 = 0;
+                ++k;
+            }
+            if (k < kPaths) load(k, j0);
+#pragma unroll
+            for (int q = 0; q < MT; ++q) {
+                const uint4* A = sw + (size_t)((k0 * MT + q) * a.ks + j00) * kStepVecs + lane;
+                float d1[NC][4], d2[NC][4];
+#pragma unroll
+                for (int j = 0; j < KS; ++j) {
+                    const uint4 a0 = A[j * kStepVecs], a1 = A[j * kStepVecs + 32], a2 = A[j * kStepVecs + 64];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const uint32_t h0 = bh[2 * j][c], h1 = bh[2 * j + 1][c];
+                        const uint32_t l0 = bl[2 * j][c], l1 = bl[2 * j + 1][c];
+                        if (j == 0) {
+                            mma16_zero(d2[c], a2, h0, h1);
+                            mma16_zero(d1[c], a0, h0, h1);
+                        } else {
+                            mma16(d2[c], a2, h0, h1);
+                            mma16(d1[c], a0, h0, h1);
+                        }
+                        mma16(d2[c], a1, l0, l1);
+                        mma16(d2[c], a1, h0, h1);
+                        mma16(d2[c], a0, l0, l1);
+                    }
+                }
+                f32x2 dr[NC], di[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    dr[c] = add2(pack2(d1[c][0], d1[c][1]), pack2(d2[c][0], d2[c][1]));
+                    di[c] = add2(pack2(d1[c][2], d1[c][3]), pack2(d2[c][2], d2[c][3]));
+                }
+                if (k0 == 0) {
+                    const f32x2 s = pack2(dinv[0], dinv[1]);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        re[q][c] = fma2(s, dr[c], re[q][c]);
+                        im[q][c] = fma2(s, di[c], im[q][c]);
+                    }
+                } else {
+#pragma unroll
+                    for (int d = 0; d < NC; ++d) {
+                        const f32x2 nd = fma2(di[d], pack2(-1.f, -1.f), 0ull);
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            re[q][c] = fma2(ur[c][d], dr[d], re[q][c]);
+                            im[q][c] = fma2(ur[c][d], di[d], im[q][c]);
+                            re[q][c] = fma2(ui[c][d], nd, re[q][c]);
+                            im[q][c] = fma2(ui[c][d], dr[d], im[q][c]);
+                        }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const uint32_t oc = tile * 8 + 2 * t + b;
+            if (oc >= cols || (b && !odd)) continue;
+            const uint32_t os = oc / um, orr = oc - os * um;
+#pragma unroll
+            for (int q = 0; q < MT; ++q) {
+                const int o = 2 * (mt0 + q) + (g >> 2);
+                if (o >= a.cout) continue;
+                float2* dst = a.out + (int64_t)o * field + (int64_t)os * slen + (int64_t)((g & 3) * NC) * m + orr;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float2 r2 = unpack2(re[q][c]), i2 = unpack2(im[q][c]);
+                    if (!odd)   // both columns: adjacent RHS of one site
+                        *reinterpret_cast<float4*>(dst + c * m) =
+                            make_float4(r2.x * winv, i2.x * winv, r2.y * winv, i2.y * winv);
+                    else
+                        dst[c * m] = make_float2((b ? r2.y : r2.x) * winv, (b ? i2.y : i2.x) * winv);
+                }
+            }
+        }
+    }
+}
+
+template <int NC, int MT, int KS>
+int layer_launch(const LayerArgs& a, cudaStream_t st) {
+    auto k = ptc_mma_kernel<NC, MT, KS>;
+    const size_t smem = (size_t)kPaths * MT * a.ks * kStepBytes;
+    if (int rc = smem_optin(reinterpret_cast<const void*>(k), smem)) return rc;
+    const int ny = a.mt / MT;
+    const int64_t tiles = (2 * a.g.vh * a.m + 7) / 8, want = (tiles + kMmaThreads / 32 - 1) / (kMmaThreads / 32);
+    const int64_t cap = sm_count() / ny > 0 ? sm_count() / ny : 1;
+    k<<<dim3((unsigned)(want < cap ? want : cap), (unsigned)ny), kMmaThreads, smem, st>>>(a);
+    QCUB_CHECK_LAUNCH();
+    return QCU_SUCCESS;
+}
+
+template <int NC>
+int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
+    switch (f.tiles * 8 + f.steps) {
+        case 8 + 1: return layer_launch<NC, 1, 1>(a, st);
+        case 8 + 2: return layer_launch<NC, 1, 2>(a, st);
+        case 8 + 4: return layer_launch<NC, 1, 4>(a, st);
+        case 16 + 1: return layer_launch<NC, 2, 1>(a, st);
+        case 16 + 2: return layer_launch<NC, 2, 2>(a, st);
+        case 16 + 4: return layer_launch<NC, 2, 4>(a, st);
+        case 32 + 1: return layer_launch<NC, 4, 1>(a, st);
+        case 32 + 2: return layer_launch<NC, 4, 2>(a, st);
+        default: return layer_launch<NC, 4, 4>(a, st);
+    }
+}
+
+// ---- weight gradient ----
+// gw[o][i][k][s'][s] = sum_{x, c, r} g_o[s'][c][r](x) conj((T_k in_i)[s][c][r](x))
+//                    = sum_{x, c, r} (U_k^dag g_o)[s'][c][r](x) conj(in_i[s][c][r](x + k)):
+// one matrix product per path over all columns.  A: rows (o, s'), K = (column, re/im) of the
+// transported gradient; B: columns (i, s, re/im), the pair (v.re, v.im) for the real part and
+// (-v.im, v.re) for the imaginary part, so a lane's D registers are whole complex numbers.
+// Both operands are split as the layer's fields, with one scale for the 8 columns of a step
+// (per operand and input channel) and first pieces of 10 bits (their products add up exactly
+// unless 16 of the K <= 64 are at the maximum at once), and all four products taken.  A step's
+// products (4 NC MMAs per tile) are accumulated from zero and added in FP32, and every
+// kFlush steps the FP32 sums go to FP64 sums in shared memory; warps, blocks and chunks are
+// summed in a fixed order.
+constexpr int kGradWarps = 8;
+constexpr int kFlush = 8;
+constexpr int kGradChunks = 16;   // blocks per path: 9 x 16 blocks of 8 warps, one per SM
+
+struct GradArgs {
+    double* part;          // [chunk][path][gridDim.z][MT CI 128]
+    const float2* gout;
+    const float2* in;
+    const float2* gauge;
+    Geom g;
+    int m, cin, cout;
+    float t_sign;
+};
+
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
+
+// MT row tiles (4 output channels each), CI input channels per block
+template <int NC, int MT, int CI>
+__global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const GradArgs a) {
+    extern __shared__ double sacc[];   // [warp][MT CI 4][lane]
+    constexpr int NA = MT * CI * 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int k = blockIdx.y, ni = (a.cin + CI - 1) / CI;
+    const int i0 = (int)(blockIdx.z % ni) * CI, o0 = (int)(blockIdx.z / ni) * MT * 4;
+    const uint32_t um = (uint32_t)a.m, cols = 2u * (uint32_t)a.g.vh * um;
+    const int m = a.m;
+    const int64_t slen = 4 * NC * (int64_t)m, field = 2 * a.g.vh * slen;
+    const bool fwd = (k & 1) != 0;
+    double* const own = sacc + (size_t)warp * NA * 32 + lane;
+    float acc[MT][CI][4];
+#pragma unroll
+    for (int q = 0; q < MT; ++q)
+#pragma unroll
+        for (int i = 0; i < CI; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[q][i][e] = 0.f;
+                own[((q * CI + i) * 4 + e) * 32] = 0.0;
+            }
+    auto flush = [&]() {
+#pragma unroll
+        for (int q = 0; q < MT; ++q)
+#pragma unroll
+            for (int i = 0; i < CI; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    own[((q * CI + i) * 4 + e) * 32] += (double)acc[q][i][e];
+                    acc[q][i][e] = 0.f;
+                }
+    };
+    int since = 0;
+#pragma unroll 1
+    for (uint32_t tile = blockIdx.x * kGradWarps + warp; tile * 8 < cols; tile += gridDim.x * kGradWarps) {
+        // this lane's columns t and t + 4: transported gradient rows g and g + 8 of every tile
+        uint32_t src[2], rr[2];
+        float2 h[MT][4][NC];
+        float mx = 0.f;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const uint32_t cw = tile * 8 + 4 * b + t;
+            const bool in_range = cw < cols;
+            const uint32_t col = in_range ? cw : cols - 1;
+            const uint32_t site = col / um;
+            rr[b] = col - site * um;
+            uint32_t link = 0;
+            bool wrap = false;
+            src[b] = site;
+            if (k) ptc_step(a.g, ptc_site(a.g, site), k, src[b], link, wrap);
+            float2 u[NC][NC];   // U_k^dag
+            if (k) {
+                const float2* U = a.gauge + (int64_t)link * (NC * NC);
+                const float sg = wrap ? a.t_sign : 1.f;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int d = 0; d < NC; ++d) {
+                        const float2 e = __ldg(U + (fwd ? d * NC + c : c * NC + d));
+                        u[c][d] = make_float2(sg * e.x, fwd ? -sg * e.y : sg * e.y);
+                    }
+            }
+#pragma unroll
+            for (int q = 0; q < MT; ++q)
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const int o = o0 + 4 * q + 2 * w + (g >> 2);
+                    const float2* gp = a.gout + (int64_t)o * field + (int64_t)site * slen + (int64_t)((g & 3) * NC) * m + rr[b];
+                    float2 v[NC];
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        v[c] = in_range && o < a.cout ? __ldg(gp + (int64_t)c * m) : make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        float2 x = make_float2(0.f, 0.f);
+                        if (k) {
+#pragma unroll
+                            for (int d = 0; d < NC; ++d) x = cfma2(u[c][d], v[d], x);
+                        } else {
+                            x = v[c];
+                        }
+                        h[q][2 * b + w][c] = x;
+                        mx = fmaxf(mx, fmaxf(fabsf(x.x), fabsf(x.y)));
+                    }
+                }
+        }
+        float ainv;
+        const float asc = scale_to_half(warp_max(mx), &ainv);
+        uint4 ah[MT][NC], al[MT][NC];
+#pragma unroll
+        for (int q = 0; q < MT; ++q)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    split16<10>(make_float2(h[q][e][c].x * asc, h[q][e][c].y * asc), hi[e], lo[e]);
+                ah[q][c] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                al[q][c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+        const float2* const v0 = a.in + (int64_t)src[0] * slen + (int64_t)((g >> 1) * NC) * m + rr[0];
+        const float2* const v1 = a.in + (int64_t)src[1] * slen + (int64_t)((g >> 1) * NC) * m + rr[1];
+        // all channels' spinors requested first (one exposed latency a step instead of CI); channels
+        // past the last are computed and not used
+        float2 xs[CI][NC][2];
+#pragma unroll
+        for (int i = 0; i < CI; ++i) {
+            const int64_t fo = (int64_t)min(i0 + i, a.cin - 1) * field;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                xs[i][c][0] = __ldg(v0 + fo + c * m);
+                xs[i][c][1] = __ldg(v1 + fo + c * m);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < CI; ++i) {
+            const float2 (&x)[NC][2] = xs[i];
+            float bx = 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) bx = fmaxf(bx, fmaxf(fabsf(x[c][b].x), fabsf(x[c][b].y)));
+            float binv;
+            const float bsc = scale_to_half(warp_max(bx), &binv);
+            uint32_t bh[NC][2], bl[NC][2];
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float re = x[c][b].x * bsc, im = x[c][b].y * bsc;
+                    split16<10>((g & 1) ? make_float2(-im, re) : make_float2(re, im), bh[c][b], bl[c][b]);
+                }
+            const float dinv = ainv * binv;
+#pragma unroll
+            for (int q = 0; q < MT; ++q) {
+                float d1[4], d2[4];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (c == 0) {
+                        mma16_zero(d2, al[q][c], bl[c][0], bl[c][1]);
+                        mma16_zero(d1, ah[q][c], bh[c][0], bh[c][1]);
+                    } else {
+                        mma16(d2, al[q][c], bl[c][0], bl[c][1]);
+                        mma16(d1, ah[q][c], bh[c][0], bh[c][1]);
+                    }
+                    mma16(d2, ah[q][c], bl[c][0], bl[c][1]);
+                    mma16(d2, al[q][c], bh[c][0], bh[c][1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[q][i][e] = fmaf(d1[e] + d2[e], dinv, acc[q][i][e]);
+            }
+        }
+        if (++since == kFlush) {
+            flush();
+            since = 0;
+        }
+    }
+    flush();
+    __syncthreads();
+    double* dst = a.part + (((size_t)blockIdx.x * kPaths + k) * gridDim.z + blockIdx.z) * (NA * 32);
+    for (int e = threadIdx.x; e < NA * 32; e += blockDim.x) {
+        double s = 0.0;
+        for (int w = 0; w < kGradWarps; ++w) s += sacc[(size_t)w * NA * 32 + e];
+        dst[e] = s;
+    }
+}
+
+// sum of the chunks, into gw
+__global__ void ptc_grad_sum_kernel(double2* __restrict__ gw, const double* __restrict__ part, int chunks, int mt, int ci,
+                                    int cin, int cout, int nz) {
+    const int na = mt * ci * 128;   // doubles of one (chunk, path, z)
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= kPaths * nz * na / 2) return;
+    const int lane = e & 31, w = (e >> 5) & 1;
+    int q = e >> 6;                 // (path, z, tile, channel)
+    const int i = q % ci; q /= ci;
+    const int tile = q % mt; q /= mt;
+    const int z = q % nz, k = q / nz;
+    const int ni = (cin + ci - 1) / ci;
+    const int ii = (z % ni) * ci + i, o = (z / ni) * mt * 4 + 4 * tile + 2 * w + (lane >> 4);
+    if (ii >= cin || o >= cout) return;
+    const double* src = part + ((size_t)k * nz + z) * na + ((tile * ci + i) * 4 + 2 * w) * 32 + lane;
+    double2 s = make_double2(0.0, 0.0);
+    for (int c = 0; c < chunks; ++c) {
+        s.x += src[(size_t)c * kPaths * nz * na];
+        s.y += src[(size_t)c * kPaths * nz * na + 32];
+    }
+    gw[(((int64_t)o * cin + ii) * kPaths + k) * 16 + ((lane >> 2) & 3) * 4 + (lane & 3)] = s;
+}
+
+struct GradShape {
+    int mt, ci, nz;
+};
+GradShape grad_shape(int cin, int cout) {
+    GradShape s;
+    s.mt = cout <= 4 ? 1 : 2;
+    s.ci = cin == 1 ? 1 : (cin <= 4 ? 4 : 8);
+    s.nz = (cin + s.ci - 1) / s.ci * ((cout + 4 * s.mt - 1) / (4 * s.mt));
+    return s;
+}
+
+template <int NC, int MT, int CI>
+int grad_launch(const GradArgs& a, double2* gw, int nz, cudaStream_t st) {
+    auto k = ptc_grad_kernel<NC, MT, CI>;
+    const size_t smem = (size_t)kGradWarps * MT * CI * 128 * sizeof(double);
+    if (int rc = smem_optin(reinterpret_cast<const void*>(k), smem)) return rc;
+    k<<<dim3(kGradChunks, kPaths, (unsigned)nz), kGradWarps * 32, smem, st>>>(a);
+    QCUB_CHECK_LAUNCH();
+    const int n = kPaths * nz * MT * CI * 64;
+    ptc_grad_sum_kernel<<<(n + 255) / 256, 256, 0, st>>>(gw, a.part, kGradChunks, MT, CI, a.cin, a.cout, nz);
+    QCUB_CHECK_LAUNCH();
+    return QCU_SUCCESS;
+}
+
+template <int NC>
+int grad_nc(const GradArgs& a, const GradShape& s, double2* gw, cudaStream_t st) {
+    switch (s.mt * 16 + s.ci) {
+        case 16 + 1: return grad_launch<NC, 1, 1>(a, gw, s.nz, st);
+        case 16 + 4: return grad_launch<NC, 1, 4>(a, gw, s.nz, st);
+        case 16 + 8: return grad_launch<NC, 1, 8>(a, gw, s.nz, st);
+        case 32 + 1: return grad_launch<NC, 2, 1>(a, gw, s.nz, st);
+        case 32 + 4: return grad_launch<NC, 2, 4>(a, gw, s.nz, st);
+        default: return grad_launch<NC, 2, 8>(a, gw, s.nz, st);
+    }
+}
+
+}  // namespace
+
+size_t ptc_grad_bytes(int cin, int cout) {
+    const GradShape s = grad_shape(cin, cout);
+    return (size_t)kGradChunks * kPaths * s.nz * s.mt * s.ci * 128 * sizeof(double);
+}
+
+int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge, const Geom& g,
+             int m, int cin, int cout, float t_sign, cudaStream_t st) {
+    const GradShape s = grad_shape(cin, cout);
+    const GradArgs a{static_cast<double*>(part), gout, in, gauge, g, m, cin, cout, t_sign};
+    switch (nc) {
+        case 2: return grad_nc<2>(a, s, gw, st);
+        case 3: return grad_nc<3>(a, s, gw, st);
+        case 4: return grad_nc<4>(a, s, gw, st);
+        default: return set_error(QCU_ERR_UNSUPPORTED, "preconditioner n_color=%d (2..4)", nc);
+    }
+}
+
+size_t ptc_frag_bytes(int cin, int cout) {
+    const FragShape f = frag_shape(cin, cout);
+    return (size_t)kPaths * f.mt * f.ks * kStepBytes + 16;
+}
+
+int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
+                cudaStream_t st) {
+    PrepArgs a{};
+    a.adj = adj;
+    for (int l = 0; l < layers; ++l) {
+        const int ci = adj ? cout[l] : cin[l], co = adj ? cin[l] : cout[l];
+        const FragShape f = frag_shape(ci, co);
+        char* base = static_cast<char*>(frag[l]);
+        a.l[l] = PrepLayer{w[l], reinterpret_cast<uint4*>(base),
+                           reinterpret_cast<float*>(base + (size_t)kPaths * f.mt * f.ks * kStepBytes), ci, co, f.mt, f.ks};
+    }
+    ptc_prepare_kernel<<<layers, 256, 0, st>>>(a);
+    QCUB_CHECK_LAUNCH();
+    return QCU_SUCCESS;
+}
+
+int ptc_layer(int nc, float2* out, const float2* in, const void* frag, const float2* gauge, const Geom& g, int m,
+              int cin, int cout, float t_sign, const int* done, cudaStream_t st) {
+    const FragShape f = frag_shape(cin, cout);
+    const char* base = static_cast<const char*>(frag);
+    const LayerArgs a{out, in, reinterpret_cast<const uint4*>(base),
+                      reinterpret_cast<const float*>(base + (size_t)kPaths * f.mt * f.ks * kStepBytes), gauge, g, m, cin, cout,
+                      f.mt, f.ks, t_sign, done};
+    switch (nc) {
+        case 2: return layer_nc<2>(a, f, st);
+        case 3: return layer_nc<3>(a, f, st);
+        case 4: return layer_nc<4>(a, f, st);
+        default: return set_error(QCU_ERR_UNSUPPORTED, "preconditioner n_color=%d (2..4)", nc);
+    }
+}
+
+}  // namespace qcub

@@ -64,6 +64,19 @@ int blocks_per_sm(const void* kernel, int block, size_t smem) {
     return per_sm;
 }
 
+int smem_optin(const void* kernel, size_t smem) {
+    if (smem <= 32 * 1024) return QCU_SUCCESS;   // fits beside the kernels' static arrays
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int dev = 0;
+    QCUB_CUDA_CHECK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_mu);
+    size_t& have = allowed[std::make_pair(kernel, dev)];
+    if (have >= smem) return QCU_SUCCESS;
+    QCUB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    have = smem;
+    return QCU_SUCCESS;
+}
+
 // ---------------- scratch ----------------
 int scratch_alloc(Scratch* s) {
     s->max_blocks = kScratchBlocks;

@@ -1,0 +1,65 @@
+"""The tensor-core layer and weight-gradient kernels of the learned preconditioner at the
+edges of their tiles: columns (site, RHS) in tiles of 8 (odd m: two sites in a lane's column
+pair; a last tile that is not full), output channels in tiles of 2 and 4, input channels in
+steps of 2 and chunks of 4 or 8, against the oracle.
+
+Tolerances: the kernels' products are exact to 2^-20 with errors of random sign, and a
+network of `layers` layers sums at most 13 x 9 x 4 of them per output, so 2e-6 holds the
+output of 2-3 layers and 4e-6 the gradient (which also carries the adjoint layers) with a
+margin of about 4 over the errors of 2^-20 sqrt(layers)."""
+import numpy as np
+import pytest
+
+import qcu_mrhs_b200 as q
+from qcu_mrhs_b200 import fields as F
+from qcu_mrhs_b200.precond import LearnedPreconditioner, identity_weights
+from tests.helpers import from_dev, rel_err, to_dev
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [((2, 2, 2, 2), 3, 1, 2, 1), ((4, 2, 2, 2), 2, 5, 2, 2), ((4, 2, 2, 4), 3, 3, 3, 5), ((2, 2, 4, 2), 4, 7, 2, 8),
+          ((4, 4, 2, 2), 3, 8, 2, 9), ((2, 4, 2, 2), 2, 9, 3, 12), ((4, 2, 4, 2), 3, 12, 2, 13), ((6, 2, 2, 2), 4, 2, 3, 4)]
+
+
+def _case(L, nc, m, layers, ch, seed, spread):
+    rng = np.random.default_rng(seed)
+    vh = F.half_volume(L)
+    ws = [w + 0.1 * (rng.standard_normal(w.shape) + 1j * rng.standard_normal(w.shape))
+          for w in identity_weights(layers, ch)]
+    ws = [w.astype(np.complex64).astype(np.complex128) for w in ws]
+    b = rng.standard_normal((2, vh, 4, nc, m)) + 1j * rng.standard_normal((2, vh, 4, nc, m))
+    # right-hand sides of very different magnitude: each column carries its own scale
+    b = (b * spread ** np.arange(m)).astype(np.complex64).astype(np.complex128)
+    return F.gauge_field(L, nc, seed + 1), ws, b
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", SHAPES)
+@pytest.mark.parametrize("spread", [1.0, 1e-3])
+def test_apply_at_tile_edges(oracle_lib, L, nc, m, layers, ch, spread):
+    g, ws, b = _case(L, nc, m, layers, ch, 100 + ch + m, spread)
+    P = LearnedPreconditioner(L, nc, m, layers, ch, t_boundary=-1.0)
+    P.set_weights(ws)
+    P.set_gauge(to_dev(g))
+    out = to_dev(np.zeros_like(b), q.SINGLE)
+    P.apply(out, to_dev(b, q.SINGLE), precision=q.SINGLE)
+    q.lib().qcuDeviceSynchronize()
+    ref = oracle_lib.precond_apply(b, ws, g, L, -1.0)
+    got = from_dev(out)
+    for j in range(m):
+        assert rel_err(got[..., j], ref[..., j]) <= 2e-6
+    P.close()
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", SHAPES)
+def test_gradient_at_tile_edges(oracle_lib, L, nc, m, layers, ch):
+    kappa = 0.12
+    g, ws, b = _case(L, nc, m, layers, ch, 200 + ch + m, 1.0)
+    P = LearnedPreconditioner(L, nc, m, layers, ch, t_boundary=-1.0)
+    P.set_weights(ws)
+    P.set_gauge(to_dev(g))
+    loss, grads = P.loss_grad(to_dev(b), kappa)
+    ref_loss, ref_grads = oracle_lib.precond_loss_grad(b, ws, g, L, kappa, -1.0)
+    assert loss == pytest.approx(ref_loss, rel=4e-6)
+    for gg, rg in zip(grads, ref_grads):
+        assert rel_err(gg, rg) <= 4e-6
+    P.close()
