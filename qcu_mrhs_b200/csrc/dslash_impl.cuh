@@ -208,17 +208,19 @@ __device__ __forceinline__ void hop_site(typename St<S>::A2 (&acc)[4][NC], const
 
 // Epilogue of one (site, RHS): store out = D in (EPI_PLAIN) or the fused combination
 // with x / r0, and add this thread's terms of the fused reductions to red.
-// `base` is the offset of (site, spin 0, colour 0, RHS) in the gathered layout.
+// `base` is the offset of (site, spin 0, colour 0, RHS) in the gathered layout; row i of x
+// (r0) is at xv[i xs] (r0[i rs]), in global or shared memory.
 template <int NC, typename S, int EPI, int NV>
 __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC], const HopParams& p,
-                                          int64_t base, typename St<S>::A2 (&red)[NV > 0 ? NV : 1]) {
+                                          int64_t base, typename St<S>::A2 (&red)[NV > 0 ? NV : 1],
+                                          const typename St<S>::S2* __restrict__ xv, int xs,
+                                          const typename St<S>::S2* __restrict__ r0,
+                                          int rs0) {
     using S2 = typename St<S>::S2;
     using A = typename St<S>::A;
     using A2 = typename St<S>::A2;
     const int m = p.m;
     S2* __restrict__ out = static_cast<S2*>(p.out);
-    const S2* __restrict__ xv = static_cast<const S2*>(p.x);
-    const S2* __restrict__ r0 = static_cast<const S2*>(p.r0);
 #pragma unroll
     for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -228,13 +230,13 @@ __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC]
             if (EPI == EPI_PLAIN) {
                 out[o] = St<S>::cv(v);
             } else {
-                const A2 xx = St<S>::ld(xv[o]);
+                const A2 xx = St<S>::ld(xv[(s * NC + c) * xs]);
                 const A a = (A)p.a;
                 A2 res;
                 if (EPI == EPI_XPAY) {
                     res = mk2<A2>(xx.x + a * v.x, xx.y + a * v.y);
                 } else if (EPI == EPI_RESID) {
-                    const A2 yy = St<S>::ld(r0[o]);
+                    const A2 yy = St<S>::ld(r0[(s * NC + c) * rs0]);
                     res = mk2<A2>(yy.x - xx.x + a * v.x, yy.y - xx.y + a * v.y);
                 } else {
                     res = mk2<A2>(xx.x - a * v.x, xx.y - a * v.y);
@@ -248,7 +250,7 @@ __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC]
                     if (EPI == EPI_RESID) {
                         red[0].x += rr.x * rr.x + rr.y * rr.y;
                     } else if (EPI == EPI_SCHUR_R0) {   // <r0, out> = sum conj(r0) out
-                        const A2 q = St<S>::ld(r0[o]);
+                        const A2 q = St<S>::ld(r0[(s * NC + c) * rs0]);
                         red[0].x += q.x * rr.x + q.y * rr.y;
                         red[0].y += q.x * rr.y - q.y * rr.x;
                     } else if (EPI == EPI_SCHUR_TS) {  // <out, x>, <out, out>
@@ -261,6 +263,15 @@ __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC]
         }
 }
 
+// the same with x and r0 read from their vectors
+template <int NC, typename S, int EPI, int NV>
+__device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC], const HopParams& p,
+                                          int64_t base, typename St<S>::A2 (&red)[NV > 0 ? NV : 1]) {
+    using S2 = typename St<S>::S2;
+    hop_store<NC, S, EPI, NV>(acc, p, base, red, static_cast<const S2*>(p.x) + base, p.m,
+                              static_cast<const S2*>(p.r0) + base, p.m);
+}
+
 // Minimum resident blocks per SM requested from the register allocator: FP64 at small N
 // otherwise takes ~190 registers (one block per SM, latency-bound); capping it at 128
 // doubles the warps in flight.  Large N keeps the compiler's choice (accumulators dominate).
@@ -269,12 +280,39 @@ struct HopMinBlocks {
     static constexpr int value = NC <= 4 ? (sizeof(S) == 8 ? 2 : 3) : 1;
 };
 
+// Epilogue vectors (x, r0) that a thread copies into its own slots of shared memory while it
+// computes the hop, up to 150 KB an SM (with at least two blocks).  Read after the hop instead,
+// their latency is exposed once per site.  <t, s>, <t, t> form (x) and <r0, v> form (x, r0), us:
+//   24^3x48, SU(3), m = 12   FP64 1187 -> 893, 1189 -> 985    FP32 -, 595 -> 460
+//   16^3x32, SU(3), m = 5    FP64 -, 119 -> 96
+//   16^4, N = 6, m = 8       FP32 169 -> 103, 165 -> 120
+// The limit leaves L1 room for the links, which all RHS of a site read: with x and r0 both
+// staged in FP64 at N = 3 (192 KB) the <r0, v> form took 1721 us.
+template <int NC, typename S, int EPI>
+struct HopStage {
+    static constexpr int kReads = EPI == EPI_PLAIN ? 0 : ((EPI == EPI_SCHUR_R0 || EPI == EPI_RESID) ? 2 : 1);
+    static constexpr int kVecBytes = 4 * NC * kRedThreads * 2 * (int)sizeof(S);   // one vector, one block
+    static constexpr int kBlocks = HopMinBlocks<NC, S>::value < 2 ? 2 : HopMinBlocks<NC, S>::value;
+    static constexpr int kFit = 150 * 1024 / (kVecBytes * kBlocks);
+    static constexpr int value = kReads < kFit ? kReads : kFit;
+};
+
+// asynchronous 4-, 8- or 16-byte copy of one complex number into shared memory
+template <typename S2>
+__device__ __forceinline__ void copy_async(S2* dst, const S2* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "n"((int)sizeof(S2))
+                 : "memory");
+}
+
 template <int NC, typename S, bool DAG, int EPI>
 __global__ void __launch_bounds__(kRedThreads, HopMinBlocks<NC, S>::value) hop_kernel(const HopParams p) {
     using S2 = typename St<S>::S2;
     using A = typename St<S>::A;
     using A2 = typename St<S>::A2;
     constexpr int NV = (EPI == EPI_SCHUR_R0 || EPI == EPI_RESID) ? 1 : (EPI == EPI_SCHUR_TS ? 2 : 0);
+    constexpr int NST = HopStage<NC, S, EPI>::value;
     if (skip_launch(p.done, p.gate)) return;
     const int m = p.m;
     const int rhs = threadIdx.x % m;
@@ -291,9 +329,28 @@ __global__ void __launch_bounds__(kRedThreads, HopMinBlocks<NC, S>::value) hop_k
     (void)total;
     for (int64_t site = ((int64_t)blockIdx.x * blockDim.x) / m + threadIdx.x / m; site < p.g.vh;
          site += site_stride) {
-        A2 acc[4][NC];
-        hop_site<NC, S, DAG>(acc, p, site, rhs);
-        hop_store<NC, S, EPI, NV>(acc, p, site * site_len + rhs, red);
+        if constexpr (NST == 0) {
+            A2 acc[4][NC];
+            hop_site<NC, S, DAG>(acc, p, site, rhs);
+            hop_store<NC, S, EPI, NV>(acc, p, site * site_len + rhs, red);
+        } else {
+            extern __shared__ __align__(16) unsigned char hop_smem[];
+            S2* const slots = reinterpret_cast<S2*>(hop_smem) + threadIdx.x;   // row i at slots[i blockDim]
+            const int64_t base = site * site_len + rhs;
+            const S2* const xv = static_cast<const S2*>(p.x) + base;
+            const S2* const r0 = static_cast<const S2*>(p.r0) + base;
+#pragma unroll
+            for (int i = 0; i < 4 * NC; ++i) copy_async(slots + i * blockDim.x, xv + i * m);
+            if constexpr (NST > 1) {
+#pragma unroll
+                for (int i = 0; i < 4 * NC; ++i) copy_async(slots + (4 * NC + i) * blockDim.x, r0 + i * m);
+            }
+            A2 acc[4][NC];
+            hop_site<NC, S, DAG>(acc, p, site, rhs);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            hop_store<NC, S, EPI, NV>(acc, p, base, red, slots, (int)blockDim.x,
+                                      NST > 1 ? slots + 4 * NC * blockDim.x : r0, NST > 1 ? (int)blockDim.x : m);
+        }
     }
     if constexpr (NV > 0) {
         double2 rv[NV];

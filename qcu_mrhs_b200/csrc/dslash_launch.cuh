@@ -36,9 +36,19 @@ int launch_hop(const HopParams& p, bool dagger, int epi, cudaStream_t stream, bo
     const int per = color_split ? NC * p.m : p.m;
     const int block = (kRedThreads / per) * per;
     const int64_t total = p.g.vh * per;
-    int grid = resident_grid(k, block, total);
+    size_t smem = 0;   // the staged epilogue vectors of hop_kernel
+    if (!color_split) {
+        switch (epi) {
+            case EPI_PLAIN: break;
+            case EPI_SCHUR_R0: case EPI_RESID: smem = HopStage<NC, S, EPI_RESID>::value; break;
+            default: smem = HopStage<NC, S, EPI_XPAY>::value;
+        }
+        smem *= (size_t)4 * NC * block * 2 * sizeof(S);
+    }
+    if (int rc = smem_optin(reinterpret_cast<const void*>(k), smem)) return rc;
+    int grid = resident_grid(k, block, total, smem);
     if (grid > kScratchBlocks) grid = kScratchBlocks;   // partial sums fit the scratch
-    k<<<grid, block, 0, stream>>>(p);
+    k<<<grid, block, smem, stream>>>(p);
     QCUB_CHECK_LAUNCH();
     return QCU_SUCCESS;
 }
