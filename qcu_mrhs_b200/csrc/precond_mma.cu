@@ -472,9 +472,14 @@ int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
 // one matrix product per path over all columns.  A: rows (o, s'), K = (column, re/im) of the
 // transported gradient; B: columns (i, s, re/im), the pair (v.re, v.im) for the real part and
 // (-v.im, v.re) for the imaginary part, so a lane's D registers are whole complex numbers.
-// Both operands are split as the layer's fields, with one scale for the 8 columns of a step
-// (per operand and input channel) and first pieces of 10 bits (their products add up exactly
-// unless 16 of the K <= 64 are at the maximum at once), and all four products taken.  A step's
+// A column is a (site, RHS) pair, and the operands' sizes run in opposite directions: the loss
+// divides by ||b_j||^2, so g goes as 1 / ||b_j|| where in goes as ||b_j||.  Every column therefore
+// takes a power of two p from its largest entries, g p and in / p (exact, and gone from the
+// product), which brings both to the square root of their product.  After that A has one scale
+// per row (o, s') and B one per input channel, each common to the 8 columns of a step: neither the
+// size of a right-hand side nor that of a channel costs bits.
+// Both operands are split as the layer's fields, with first pieces of 10 bits (their products add
+// up exactly unless 16 of the K <= 64 are at the maximum at once), and all four products taken.  A step's
 // products (4 NC MMAs per tile) are accumulated from zero and added in FP32, and every
 // kFlush steps the FP32 sums go to FP64 sums in shared memory; warps, blocks and chunks are
 // summed in a fixed order.
@@ -492,6 +497,25 @@ struct GradArgs {
     float t_sign;
 };
 
+// power of two nearest to sqrt(x / h) for a column's largest entries h and x, and its inverse
+__device__ __forceinline__ float balance(float h, float x, float* inv) {
+    const int d = ((int)(__float_as_uint(x) >> 23) - (int)(__float_as_uint(h) >> 23)) >> 1;
+    const int c = min(max(d, -126), 126);
+    *inv = __uint_as_float((uint32_t)(127 - c) << 23);
+    return __uint_as_float((uint32_t)(127 + c) << 23);
+}
+__device__ __forceinline__ float finite_abs(float v) { return fabsf(v) <= 3.4028235e38f ? fabsf(v) : 0.f; }
+
+// maximum over the 8 lanes of one column pair (t), and over the 4 lanes of one row (g)
+__device__ __forceinline__ float column_max(float v) {
+#pragma unroll
+    for (int off = 16; off >= 4; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
+__device__ __forceinline__ float row_max(float v) {
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
@@ -538,7 +562,6 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
         // this lane's columns t and t + 4: transported gradient rows g and g + 8 of every tile
         uint32_t src[2], rr[2];
         float2 h[MT][4][NC];
-        float mx = 0.f;
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const uint32_t cw = tile * 8 + 4 * b + t;
@@ -582,24 +605,9 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                             x = v[c];
                         }
                         h[q][2 * b + w][c] = x;
-                        mx = fmaxf(mx, fmaxf(fabsf(x.x), fabsf(x.y)));
                     }
                 }
         }
-        float ainv;
-        const float asc = scale_to_half(warp_max(mx), &ainv);
-        uint4 ah[MT][NC], al[MT][NC];
-#pragma unroll
-        for (int q = 0; q < MT; ++q)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                uint32_t hi[4], lo[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    split16<10>(make_float2(h[q][e][c].x * asc, h[q][e][c].y * asc), hi[e], lo[e]);
-                ah[q][c] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                al[q][c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            }
         const float2* const v0 = a.in + (int64_t)src[0] * slen + (int64_t)((g >> 1) * NC) * m + rr[0];
         const float2* const v1 = a.in + (int64_t)src[1] * slen + (int64_t)((g >> 1) * NC) * m + rr[1];
         // all channels' spinors requested first (one exposed latency a step instead of CI); channels
@@ -614,14 +622,83 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                 xs[i][c][1] = __ldg(v1 + fo + c * m);
             }
         }
+        // the columns' powers of two
+        float pc[2], pi[2];
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            float hm = 0.f, xm = 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+#pragma unroll
+                for (int q = 0; q < MT; ++q)
+#pragma unroll
+                    for (int w = 0; w < 2; ++w)
+                        hm = fmaxf(hm, fmaxf(fabsf(h[q][2 * b + w][c].x), fabsf(h[q][2 * b + w][c].y)));
+#pragma unroll
+                for (int i = 0; i < CI; ++i) xm = fmaxf(xm, fmaxf(fabsf(xs[i][c][b].x), fabsf(xs[i][c][b].y)));
+            }
+            hm = column_max(hm);
+            xm = column_max(xm);
+            // an infinity (of one channel) does not decide over the other channels' bits
+            if (__any_sync(0xffffffffu, fmaxf(hm, xm) > 3.4028235e38f)) {
+                hm = xm = 0.f;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+#pragma unroll
+                    for (int q = 0; q < MT; ++q)
+#pragma unroll
+                        for (int w = 0; w < 2; ++w)
+                            hm = fmaxf(hm, fmaxf(finite_abs(h[q][2 * b + w][c].x), finite_abs(h[q][2 * b + w][c].y)));
+#pragma unroll
+                    for (int i = 0; i < CI; ++i)
+                        xm = fmaxf(xm, fmaxf(finite_abs(xs[i][c][b].x), finite_abs(xs[i][c][b].y)));
+                }
+                hm = column_max(hm);
+                xm = column_max(xm);
+            }
+            pc[b] = balance(hm, xm, &pi[b]);
+        }
+        float ainv[MT][2];
+        uint4 ah[MT][NC], al[MT][NC];
+#pragma unroll
+        for (int q = 0; q < MT; ++q) {
+            float asc[2];
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                float mx = 0.f;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        float2& v = h[q][2 * b + w][c];
+                        v.x *= pc[b];
+                        v.y *= pc[b];
+                        mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
+                    }
+                asc[w] = scale_to_half(row_max(mx), &ainv[q][w]);
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    split16<10>(make_float2(h[q][e][c].x * asc[e & 1], h[q][e][c].y * asc[e & 1]), hi[e], lo[e]);
+                ah[q][c] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                al[q][c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < CI; ++i) {
-            const float2 (&x)[NC][2] = xs[i];
+            float2 (&x)[NC][2] = xs[i];
             float bx = 0.f;
 #pragma unroll
             for (int c = 0; c < NC; ++c)
 #pragma unroll
-                for (int b = 0; b < 2; ++b) bx = fmaxf(bx, fmaxf(fabsf(x[c][b].x), fabsf(x[c][b].y)));
+                for (int b = 0; b < 2; ++b) {
+                    x[c][b].x *= pi[b];
+                    x[c][b].y *= pi[b];
+                    bx = fmaxf(bx, fmaxf(fabsf(x[c][b].x), fabsf(x[c][b].y)));
+                }
             float binv;
             const float bsc = scale_to_half(warp_max(bx), &binv);
             uint32_t bh[NC][2], bl[NC][2];
@@ -632,9 +709,9 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                     const float re = x[c][b].x * bsc, im = x[c][b].y * bsc;
                     split16<10>((g & 1) ? make_float2(-im, re) : make_float2(re, im), bh[c][b], bl[c][b]);
                 }
-            const float dinv = ainv * binv;
 #pragma unroll
             for (int q = 0; q < MT; ++q) {
+                const float dinv[2] = {ainv[q][0] * binv, ainv[q][1] * binv};   // of rows g and g + 8
                 float d1[4], d2[4];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -649,7 +726,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                     mma16(d2, al[q][c], bh[c][0], bh[c][1]);
                 }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[q][i][e] = fmaf(d1[e] + d2[e], dinv, acc[q][i][e]);
+                for (int e = 0; e < 4; ++e) acc[q][i][e] = fmaf(d1[e] + d2[e], dinv[e >> 1], acc[q][i][e]);
             }
         }
         if (++since == kFlush) {

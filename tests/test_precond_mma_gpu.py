@@ -63,3 +63,27 @@ def test_gradient_at_tile_edges(oracle_lib, L, nc, m, layers, ch):
     for gg, rg in zip(grads, ref_grads):
         assert rel_err(gg, rg) <= 4e-6
     P.close()
+
+
+def _loss_grad(L, nc, m, layers, ch, g, ws, b, kappa):
+    P = LearnedPreconditioner(L, nc, m, layers, ch, t_boundary=-1.0)
+    P.set_weights(ws)
+    P.set_gauge(to_dev(g))
+    loss, grads = P.loss_grad(to_dev(b), kappa)
+    P.close()
+    return loss, grads
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", [s for s in SHAPES if s[2] > 1])
+@pytest.mark.parametrize("spread,period", [(1e-3, 2), (1e-6, 2), (1e-2, 4)])
+def test_gradient_of_unequal_right_hand_sides(oracle_lib, L, nc, m, layers, ch, spread, period):
+    """The loss divides by each right-hand side's norm: small ones have large output gradients, and
+    all of them count alike in the weight gradient."""
+    kappa = 0.12
+    g, ws, b = _case(L, nc, m, layers, ch, 300 + ch + m, 1.0)
+    b = (b * spread ** (np.arange(m) % period)).astype(np.complex64).astype(np.complex128)
+    loss, grads = _loss_grad(L, nc, m, layers, ch, g, ws, b, kappa)
+    ref_loss, ref_grads = oracle_lib.precond_loss_grad(b, ws, g, L, kappa, -1.0)
+    assert loss == pytest.approx(ref_loss, rel=4e-6)
+    for gg, rg in zip(grads, ref_grads):
+        assert rel_err(gg, rg) <= 4e-6
