@@ -72,6 +72,33 @@ __device__ __forceinline__ void split16(float2 v, uint32_t& hi, uint32_t& lo) {
     hi = half_bits(__float22half2_rn(f));   // exact
     lo = half_bits(__floats2half2_rn(v.x - f.x, v.y - f.y));
 }
+// Operands at all 24 bits.  With a = a0 + ra and x = x0 + rx (a0, x0 the first pieces),
+//   a x = a0 x0 + a0 rx + ra x:
+// ra and rx as two FP16 pieces each, times 2^9 (kRest brings the products back) so that they stay
+// clear of FP16's subnormal numbers, and x itself as two floating-point pieces.  What is lost of
+// an entry is below 2^-23 of itself or 2^-48 of the largest entry under its scale.
+constexpr float kRestUp = 512.f, kRest = 1.f / 512.f;
+__device__ __forceinline__ void split_float(float2 v, uint32_t& h, uint32_t& l) {   // v = h + l
+    const __half2 b = __float22half2_rn(v);
+    const float2 e = __half22float2(b);
+    h = half_bits(b);
+    l = half_bits(__floats2half2_rn(v.x - e.x, v.y - e.y));
+}
+// first piece and 2^9 times the rest in two pieces of the pair v (scaled)
+__device__ __forceinline__ void split_rest(float2 v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    const float2 f = make_float2(round_first<9>(v.x), round_first<9>(v.y));
+    p0 = half_bits(__float22half2_rn(f));   // exact
+    split_float(make_float2((v.x - f.x) * kRestUp, (v.y - f.y) * kRestUp), p1, p2);
+}
+struct Pieces {
+    uint32_t p0, p1, p2, h, l;
+};
+__device__ __forceinline__ Pieces split_field(float2 v) {
+    Pieces r;
+    split_rest(v, r.p0, r.p1, r.p2);
+    split_float(v, r.h, r.l);
+    return r;
+}
 // three FP16 pairs
 __device__ __forceinline__ void split16x3(float2 v, uint32_t& h0, uint32_t& h1, uint32_t& h2) {
     const float2 f = make_float2(round_first<9>(v.x), round_first<9>(v.y)), r = make_float2(v.x - f.x, v.y - f.y);
@@ -478,13 +505,10 @@ int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
 // product), which brings both to the square root of their product.  After that A has one scale
 // per row (o, s') and B one per input channel, each common to the 8 columns of a step: neither the
 // size of a right-hand side nor that of a channel costs bits.
-// Both operands are split as the layer's fields, with first pieces of 10 bits (their products add
-// up exactly unless 16 of the K <= 64 are at the maximum at once), and all four products taken.  A step's
-// products (4 NC MMAs per tile) are accumulated from zero and added in FP32, and every
-// kFlush steps the FP32 sums go to FP64 sums in shared memory; warps, blocks and chunks are
-// summed in a fixed order.
+// Both operands keep 24 bits (split_rest): the first pieces' products add up exactly (K <= 64), the
+// other five go to a second accumulator.  A step's products (6 NC MMAs per tile, one rounding)
+// are added to FP64 sums in shared memory; warps, blocks and chunks are summed in a fixed order.
 constexpr int kGradWarps = 8;
-constexpr int kFlush = 8;
 constexpr int kGradChunks = 16;   // blocks per path: 9 x 16 blocks of 8 warps, one per SM
 
 struct GradArgs {
@@ -535,28 +559,8 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
     const int64_t slen = 4 * NC * (int64_t)m, field = 2 * a.g.vh * slen;
     const bool fwd = (k & 1) != 0;
     double* const own = sacc + (size_t)warp * NA * 32 + lane;
-    float acc[MT][CI][4];
 #pragma unroll
-    for (int q = 0; q < MT; ++q)
-#pragma unroll
-        for (int i = 0; i < CI; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                acc[q][i][e] = 0.f;
-                own[((q * CI + i) * 4 + e) * 32] = 0.0;
-            }
-    auto flush = [&]() {
-#pragma unroll
-        for (int q = 0; q < MT; ++q)
-#pragma unroll
-            for (int i = 0; i < CI; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    own[((q * CI + i) * 4 + e) * 32] += (double)acc[q][i][e];
-                    acc[q][i][e] = 0.f;
-                }
-    };
-    int since = 0;
+    for (int e = 0; e < NA; ++e) own[e * 32] = 0.0;
 #pragma unroll 1
     for (uint32_t tile = blockIdx.x * kGradWarps + warp; tile * 8 < cols; tile += gridDim.x * kGradWarps) {
         // this lane's columns t and t + 4: transported gradient rows g and g + 8 of every tile
@@ -659,7 +663,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
             pc[b] = balance(hm, xm, &pi[b]);
         }
         float ainv[MT][2];
-        uint4 ah[MT][NC], al[MT][NC];
+        uint4 a0[MT][NC], a1[MT][NC], a2[MT][NC];
 #pragma unroll
         for (int q = 0; q < MT; ++q) {
             float asc[2];
@@ -679,12 +683,13 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                uint32_t hi[4], lo[4];
+                uint32_t p0[4], p1[4], p2[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    split16<10>(make_float2(h[q][e][c].x * asc[e & 1], h[q][e][c].y * asc[e & 1]), hi[e], lo[e]);
-                ah[q][c] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                al[q][c] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    split_rest(make_float2(h[q][e][c].x * asc[e & 1], h[q][e][c].y * asc[e & 1]), p0[e], p1[e], p2[e]);
+                a0[q][c] = make_uint4(p0[0], p0[1], p0[2], p0[3]);
+                a1[q][c] = make_uint4(p1[0], p1[1], p1[2], p1[3]);
+                a2[q][c] = make_uint4(p2[0], p2[1], p2[2], p2[3]);
             }
         }
 #pragma unroll
@@ -701,13 +706,13 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                 }
             float binv;
             const float bsc = scale_to_half(warp_max(bx), &binv);
-            uint32_t bh[NC][2], bl[NC][2];
+            Pieces y[NC][2];
 #pragma unroll
             for (int c = 0; c < NC; ++c)
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const float re = x[c][b].x * bsc, im = x[c][b].y * bsc;
-                    split16<10>((g & 1) ? make_float2(-im, re) : make_float2(re, im), bh[c][b], bl[c][b]);
+                    y[c][b] = split_field((g & 1) ? make_float2(-im, re) : make_float2(re, im));
                 }
 #pragma unroll
             for (int q = 0; q < MT; ++q) {
@@ -715,26 +720,25 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                 float d1[4], d2[4];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
+                    const Pieces &u = y[c][0], &v = y[c][1];
                     if (c == 0) {
-                        mma16_zero(d2, al[q][c], bl[c][0], bl[c][1]);
-                        mma16_zero(d1, ah[q][c], bh[c][0], bh[c][1]);
+                        mma16_zero(d2, a2[q][c], u.h, v.h);
+                        mma16_zero(d1, a0[q][c], u.p0, v.p0);
                     } else {
-                        mma16(d2, al[q][c], bl[c][0], bl[c][1]);
-                        mma16(d1, ah[q][c], bh[c][0], bh[c][1]);
+                        mma16(d2, a2[q][c], u.h, v.h);
+                        mma16(d1, a0[q][c], u.p0, v.p0);
                     }
-                    mma16(d2, ah[q][c], bl[c][0], bl[c][1]);
-                    mma16(d2, al[q][c], bh[c][0], bh[c][1]);
+                    mma16(d2, a0[q][c], u.p2, v.p2);
+                    mma16(d2, a1[q][c], u.l, v.l);
+                    mma16(d2, a0[q][c], u.p1, v.p1);
+                    mma16(d2, a1[q][c], u.h, v.h);
                 }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[q][i][e] = fmaf(d1[e] + d2[e], dinv[e >> 1], acc[q][i][e]);
+                for (int e = 0; e < 4; ++e)
+                    own[((q * CI + i) * 4 + e) * 32] += (double)(fmaf(d2[e], kRest, d1[e]) * dinv[e >> 1]);
             }
         }
-        if (++since == kFlush) {
-            flush();
-            since = 0;
-        }
     }
-    flush();
     __syncthreads();
     double* dst = a.part + (((size_t)blockIdx.x * kPaths + k) * gridDim.z + blockIdx.z) * (NA * 32);
     for (int e = threadIdx.x; e < NA * 32; e += blockDim.x) {

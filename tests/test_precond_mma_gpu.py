@@ -87,3 +87,16 @@ def test_gradient_of_unequal_right_hand_sides(oracle_lib, L, nc, m, layers, ch, 
     assert loss == pytest.approx(ref_loss, rel=4e-6)
     for gg, rg in zip(grads, ref_grads):
         assert rel_err(gg, rg) <= 4e-6
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", SHAPES)
+def test_gradient_of_unequal_spins(oracle_lib, L, nc, m, layers, ch):
+    """Spin s of the input is a column of its own in the first layer's gradient: small spins to the
+    tolerance of the large one."""
+    kappa = 0.12
+    g, ws, b = _case(L, nc, m, layers, ch, 500 + ch + m, 1.0)
+    b = (b * np.array([1.0, 1e-2, 1e-3, 1e-4])[:, None, None]).astype(np.complex64).astype(np.complex128)
+    _, grads = _loss_grad(L, nc, m, layers, ch, g, ws, b, kappa)
+    _, ref_grads = oracle_lib.precond_loss_grad(b, ws, g, L, kappa, -1.0)
+    for s in range(4):
+        assert rel_err(grads[0][..., s], ref_grads[0][..., s]) <= 4e-6
