@@ -7,20 +7,23 @@
 //
 // FP32 products on the 16-bit MMA (mma.sync m16n8k16, FP32 accumulation): operands are scaled
 // by powers of two so that their largest entries sit at 2^14 (the weights per layer, every
-// column of a field per path), split into FP16 pieces, and the pieces' products accumulated.
-//   first piece  the value rounded to a multiple of 2^6, so 9 bits of the largest entry.  Products
-//                of two first pieces are multiples of 2^12 below 2^30, and 64 of them (the K of a
-//                path) add up within 24 bits: exact.
-//   the rest     weights w = w0 + w1 + w2 (w1, w2 of 11 bits each: all 24 bits), fields
-//                x = x0 + x1 (x1 = fp16(x - x0), an error of random sign below 2^-22 of the largest
-//                entry); w0 x1 + w1 x0 + w2 x0 + w1 x1.
+// column of a field per path) and split into FP16 pieces.
+//   first pieces  w0, x0: the values rounded to multiples of 2^6, so 9 bits of the largest entry.
+//                 Products of two of them are multiples of 2^12 up to 2^30, and 64 of them (the
+//                 largest K that one accumulator sees) add up within 24 bits: exact.
+//   the rest      w x = w0 x0 + w0 (x - x0) + (w - w0) x, with x - x0 = (x1 + x2) / 2^9,
+//                 w - w0 = (w1 + w2) / 2^9 and x = h + l: w0 x1 + w0 x2 + w1 h + w1 l + w2 h, five
+//                 more products.  The factor 2^9 keeps the pieces clear of FP16's subnormal
+//                 numbers.  What is lost of an entry is below 2^-23 of itself, or 2^-48 of the
+//                 largest entry under its scale: FP32's own precision.
 // The exactness of the first product matters because the MMA truncates: it keeps 2 bits
 // below FP32's last place of the largest addend and rounds the sum toward zero (measured: with
-// 11-bit pieces a sum over K = 64 is short by 9e-8 of itself on average).  That bias and what is
-// lost of the weights are the same at every site, so they add up in the weight gradient:
-// 1.1e-6 of it, against 3.5e-8 with FP32 arithmetic.  One path's product is accumulated from
-// zero and added to the FP32 result outside the MMA, so the sums are chains of at most 9 FP32
-// additions.
+// 11-bit pieces a sum over K = 64 is short by 9e-8 of itself on average).  That bias is the same at
+// every site, so it adds up in the weight gradient: 1.1e-6 of it, against 3.5e-8 with FP32
+// arithmetic.  The five small products are truncated 2^-9 lower.  The sums of one step (a path, up
+// to 4 input channels) are accumulated from zero and added to the FP32 result outside the MMA with
+// one rounding, so an output is a chain of 2 N FMAs a link path and step, 16 N + 1 for up to 4
+// input channels.
 //
 // Fragments (PTX ISA, mma.m16n8k16): lane 4 g + t holds A rows g, g + 8 at K 2t..2t+1 and
 // 2t+8..2t+9, B column g at the same K, D rows g, g + 8 at columns 2t, 2t + 1.  K-step j holds
@@ -58,25 +61,13 @@ __device__ __forceinline__ void mma16_zero(float (&d)[4], const uint4& a, uint32
 
 __device__ __forceinline__ uint32_t half_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 
-// v (below 2^15) rounded to a multiple of 2^(15 - BITS): adding 1.5 x 2^(38 - BITS) leaves no
-// lower bits
-template <int BITS>
+// v (below 2^15) rounded to a multiple of 2^6: adding 1.5 x 2^29 leaves no lower bits
 __device__ __forceinline__ float round_first(float v) {
-    constexpr float c = 1.5f * (float)(1ull << (38 - BITS));
+    constexpr float c = 1.5f * (float)(1 << 29);
     return __fadd_rn(__fadd_rn(v, c), -c);
 }
-// first (BITS bits) and second FP16 pair of the pair v (scaled)
-template <int BITS>
-__device__ __forceinline__ void split16(float2 v, uint32_t& hi, uint32_t& lo) {
-    const float2 f = make_float2(round_first<BITS>(v.x), round_first<BITS>(v.y));
-    hi = half_bits(__float22half2_rn(f));   // exact
-    lo = half_bits(__floats2half2_rn(v.x - f.x, v.y - f.y));
-}
-// Operands at all 24 bits.  With a = a0 + ra and x = x0 + rx (a0, x0 the first pieces),
-//   a x = a0 x0 + a0 rx + ra x:
-// ra and rx as two FP16 pieces each, times 2^9 (kRest brings the products back) so that they stay
-// clear of FP16's subnormal numbers, and x itself as two floating-point pieces.  What is lost of
-// an entry is below 2^-23 of itself or 2^-48 of the largest entry under its scale.
+
+// 2^9 on the rest's pieces, and what brings their products back
 constexpr float kRestUp = 512.f, kRest = 1.f / 512.f;
 __device__ __forceinline__ void split_float(float2 v, uint32_t& h, uint32_t& l) {   // v = h + l
     const __half2 b = __float22half2_rn(v);
@@ -86,7 +77,7 @@ __device__ __forceinline__ void split_float(float2 v, uint32_t& h, uint32_t& l) 
 }
 // first piece and 2^9 times the rest in two pieces of the pair v (scaled)
 __device__ __forceinline__ void split_rest(float2 v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    const float2 f = make_float2(round_first<9>(v.x), round_first<9>(v.y));
+    const float2 f = make_float2(round_first(v.x), round_first(v.y));
     p0 = half_bits(__float22half2_rn(f));   // exact
     split_float(make_float2((v.x - f.x) * kRestUp, (v.y - f.y) * kRestUp), p1, p2);
 }
@@ -98,15 +89,6 @@ __device__ __forceinline__ Pieces split_field(float2 v) {
     split_rest(v, r.p0, r.p1, r.p2);
     split_float(v, r.h, r.l);
     return r;
-}
-// three FP16 pairs
-__device__ __forceinline__ void split16x3(float2 v, uint32_t& h0, uint32_t& h1, uint32_t& h2) {
-    const float2 f = make_float2(round_first<9>(v.x), round_first<9>(v.y)), r = make_float2(v.x - f.x, v.y - f.y);
-    const __half2 b = __float22half2_rn(r);
-    const float2 e = __half22float2(b);
-    h0 = half_bits(__float22half2_rn(f));
-    h1 = half_bits(b);
-    h2 = half_bits(__floats2half2_rn(r.x - e.x, r.y - e.y));
 }
 
 // power of two that brings a maximum m into [2^14, 2^15), and its inverse
@@ -127,7 +109,7 @@ struct FragShape {
 
 FragShape frag_shape(int cin, int cout) {
     FragShape s;
-    s.steps = cin <= 2 ? 1 : (cin <= 4 ? 2 : (cin <= 8 ? 4 : 2));
+    s.steps = cin <= 2 ? 1 : 2;
     s.ks = (cin + 2 * s.steps - 1) / (2 * s.steps) * s.steps;
     s.tiles = cout <= 2 ? 1 : (cout <= 4 ? 2 : 4);
     if (s.tiles == 4 && (size_t)kPaths * 4 * s.ks * kStepBytes > 224 * 1024) s.tiles = 2;
@@ -185,8 +167,8 @@ __global__ void ptc_prepare_kernel(PrepArgs a) {
             }
             v.x *= sc;
             v.y *= sc;
-            split16x3(make_float2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
-            split16x3(make_float2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
+            split_rest(make_float2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
+            split_rest(make_float2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
         }
         uint4* f = L.frag + (int64_t)(e >> 5) * kStepVecs + lane;
         f[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
@@ -281,16 +263,14 @@ __device__ __forceinline__ float2 cfma2(float2 a, float2 b, float2 c) {   // c +
 }
 
 // One warp per tile of 8 consecutive columns (site, RHS) of the flattened full lattice, all
-// colours, 2 MT output channels.  The block's weights (its MT row tiles) stay in shared memory
-// (216 KB for 8 x 8 channels), so one block of 8 warps runs on an SM, at 255 registers: a
-// step's spinors and link are requested under the products of the step before it.  16^4,
-// SU(3), m = 8, one 8 -> 8 layer: 7.0 ms as FP32 arithmetic with a thread per (site, output
-// channel, RHS), each transporting every input again; 2.07 ms with 12 warps and no prefetch;
-// 1.85 ms so.  5 MT KS NC = 240 MMAs a path bound it at 1.05 ms; the rest is latency that 8
-// warps do not cover.
+// colours, 2 MT output channels, input channels 2 KS at a time.  The block's weights (its MT row
+// tiles) stay in shared memory (216 KB for 8 x 8 channels), so one block of 8 warps runs on an SM, at
+// up to 255 registers: a step's spinors and link are requested under the products of the step
+// before it.
 template <int NC, int MT, int KS>
 __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs a) {
     if (a.done != nullptr && *a.done) return;
+    constexpr int CG = NC == 4 && KS > 1 ? 2 : NC;
     extern __shared__ uint4 sw[];
     const int mt0 = blockIdx.y * MT;
     const int per_path = MT * a.ks * kStepVecs;
@@ -324,26 +304,29 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
         uint32_t link = 0;
         bool wrap = false;
         float2 u0[NC][NC];   // link of column 2t, as stored (transposed for backward paths)
-        auto load = [&](int k, int j0) {
+        auto step = [&](int k) {   // base of path k's spinors
             uint32_t src = site;
-            if (k) {
-                ptc_step(a.g, ps, k, src, link, wrap);
-                const float2* U = a.gauge + (int64_t)__shfl_sync(0xffffffffu, link, 8 * t) * (NC * NC);
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-#pragma unroll
-                    for (int d = 0; d < NC; ++d) u0[c][d] = __ldg(U + ((k & 1) ? c * NC + d : d * NC + c));
-            }
-            const float2* v = in + (int64_t)src * slen;
-#pragma unroll
-            for (int i = 0; i < 2 * KS; ++i) {
-                // channels past the last meet zero weights: any finite number of the field will do
-                const float2* vi = v + (int64_t)min(2 * j0 + i, a.cin - 1) * field;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) x[i][c] = __ldg(vi + c * m);
-            }
+            if (k) ptc_step(a.g, ps, k, src, link, wrap);
+            return in + (int64_t)src * slen;
         };
-        load(0, 0);
+        auto load_link = [&](int k) {
+            if (k == 0) return;
+            const float2* U = a.gauge + (int64_t)__shfl_sync(0xffffffffu, link, 8 * t) * (NC * NC);
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+                for (int d = 0; d < NC; ++d) u0[c][d] = __ldg(U + ((k & 1) ? c * NC + d : d * NC + c));
+        };
+        // channels past the last meet zero weights: any finite number of the field will do
+        auto load_colour = [&](const float2* v, int j0, int c) {
+#pragma unroll
+            for (int i = 0; i < 2 * KS; ++i) x[i][c] = __ldg(v + (int64_t)min(2 * j0 + i, a.cin - 1) * field + c * m);
+        };
+        {
+            const float2* v = step(0);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) load_colour(v, 0, c);
+        }
 #pragma unroll 1
         for (int k = 0, j0 = 0; k < kPaths;) {
             float mx = 0.f;
@@ -355,12 +338,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             float inv;
             const float sc = scale_to_half(mx, &inv);
-            uint32_t bh[2 * KS][NC], bl[2 * KS][NC];
-#pragma unroll
-            for (int i = 0; i < 2 * KS; ++i)
-#pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    split16<9>(make_float2(x[i][c].x * sc, x[i][c].y * sc), bh[i][c], bl[i][c]);
             // scale, link and boundary of this lane's D columns 2t and 2t + 1; the scale goes into
             // the link
             float dinv[2];
@@ -389,53 +366,67 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
                 j0 = 0;
                 ++k;
             }
-            if (k < kPaths) load(k, j0);
+            const bool more = k < kPaths;
+            const float2* next = in;
+            if (more) {
+                next = step(k);
+                if (j0 == 0) load_link(k);
+            }
+            // CG colours at a time: their pieces, then the next step's spinors into the registers that
+            // the pieces leave, then the products
 #pragma unroll
-            for (int q = 0; q < MT; ++q) {
-                const uint4* A = sw + (size_t)((k0 * MT + q) * a.ks + j00) * kStepVecs + lane;
-                float d1[NC][4], d2[NC][4];
+            for (int c0 = 0; c0 < NC; c0 += CG) {
+                Pieces y[2 * KS][CG];
 #pragma unroll
-                for (int j = 0; j < KS; ++j) {
-                    const uint4 a0 = A[j * kStepVecs], a1 = A[j * kStepVecs + 32], a2 = A[j * kStepVecs + 64];
+                for (int i = 0; i < 2 * KS; ++i)
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const uint32_t h0 = bh[2 * j][c], h1 = bh[2 * j + 1][c];
-                        const uint32_t l0 = bl[2 * j][c], l1 = bl[2 * j + 1][c];
-                        if (j == 0) {
-                            mma16_zero(d2[c], a2, h0, h1);
-                            mma16_zero(d1[c], a0, h0, h1);
-                        } else {
-                            mma16(d2[c], a2, h0, h1);
-                            mma16(d1[c], a0, h0, h1);
+                    for (int c = 0; c < CG; ++c)
+                        y[i][c] = split_field(make_float2(x[i][c0 + c].x * sc, x[i][c0 + c].y * sc));
+                if (more) {
+#pragma unroll
+                    for (int c = 0; c < CG; ++c) load_colour(next, j0, c0 + c);
+                }
+#pragma unroll
+                for (int q = 0; q < MT; ++q) {
+                    const uint4* A = sw + (size_t)((k0 * MT + q) * a.ks + j00) * kStepVecs + lane;
+                    float d1[CG][4], d2[CG][4];
+#pragma unroll
+                    for (int j = 0; j < KS; ++j) {
+                        const uint4 a0 = A[j * kStepVecs], a1 = A[j * kStepVecs + 32], a2 = A[j * kStepVecs + 64];
+#pragma unroll
+                        for (int c = 0; c < CG; ++c) {
+                            const Pieces &u = y[2 * j][c], &v = y[2 * j + 1][c];
+                            if (j == 0) {
+                                mma16_zero(d2[c], a2, u.h, v.h);
+                                mma16_zero(d1[c], a0, u.p0, v.p0);
+                            } else {
+                                mma16(d2[c], a2, u.h, v.h);
+                                mma16(d1[c], a0, u.p0, v.p0);
+                            }
+                            mma16(d2[c], a0, u.p2, v.p2);
+                            mma16(d2[c], a1, u.l, v.l);
+                            mma16(d2[c], a0, u.p1, v.p1);
+                            mma16(d2[c], a1, u.h, v.h);
                         }
-                        mma16(d2[c], a1, l0, l1);
-                        mma16(d2[c], a1, h0, h1);
-                        mma16(d2[c], a0, l0, l1);
                     }
-                }
-                f32x2 dr[NC], di[NC];
+                    const f32x2 kr = pack2(kRest, kRest);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    dr[c] = add2(pack2(d1[c][0], d1[c][1]), pack2(d2[c][0], d2[c][1]));
-                    di[c] = add2(pack2(d1[c][2], d1[c][3]), pack2(d2[c][2], d2[c][3]));
-                }
-                if (k0 == 0) {
-                    const f32x2 s = pack2(dinv[0], dinv[1]);
+                    for (int c = 0; c < CG; ++c) {
+                        const f32x2 dr = fma2(pack2(d2[c][0], d2[c][1]), kr, pack2(d1[c][0], d1[c][1]));
+                        const f32x2 di = fma2(pack2(d2[c][2], d2[c][3]), kr, pack2(d1[c][2], d1[c][3]));
+                        if (k0 == 0) {
+                            const f32x2 s = pack2(dinv[0], dinv[1]);
+                            re[q][c0 + c] = fma2(s, dr, re[q][c0 + c]);
+                            im[q][c0 + c] = fma2(s, di, im[q][c0 + c]);
+                        } else {
+                            const f32x2 nd = fma2(di, pack2(-1.f, -1.f), 0ull);
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        re[q][c] = fma2(s, dr[c], re[q][c]);
-                        im[q][c] = fma2(s, di[c], im[q][c]);
-                    }
-                } else {
-#pragma unroll
-                    for (int d = 0; d < NC; ++d) {
-                        const f32x2 nd = fma2(di[d], pack2(-1.f, -1.f), 0ull);
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            re[q][c] = fma2(ur[c][d], dr[d], re[q][c]);
-                            im[q][c] = fma2(ur[c][d], di[d], im[q][c]);
-                            re[q][c] = fma2(ui[c][d], nd, re[q][c]);
-                            im[q][c] = fma2(ui[c][d], dr[d], im[q][c]);
+                            for (int r = 0; r < NC; ++r) {
+                                re[q][r] = fma2(ur[r][c0 + c], dr, re[q][r]);
+                                im[q][r] = fma2(ur[r][c0 + c], di, im[q][r]);
+                                re[q][r] = fma2(ui[r][c0 + c], nd, re[q][r]);
+                                im[q][r] = fma2(ui[r][c0 + c], dr, im[q][r]);
+                            }
                         }
                     }
                 }
@@ -480,16 +471,13 @@ int layer_launch(const LayerArgs& a, cudaStream_t st) {
 
 template <int NC>
 int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
-    switch (f.tiles * 8 + f.steps) {
-        case 8 + 1: return layer_launch<NC, 1, 1>(a, st);
-        case 8 + 2: return layer_launch<NC, 1, 2>(a, st);
-        case 8 + 4: return layer_launch<NC, 1, 4>(a, st);
-        case 16 + 1: return layer_launch<NC, 2, 1>(a, st);
-        case 16 + 2: return layer_launch<NC, 2, 2>(a, st);
-        case 16 + 4: return layer_launch<NC, 2, 4>(a, st);
-        case 32 + 1: return layer_launch<NC, 4, 1>(a, st);
-        case 32 + 2: return layer_launch<NC, 4, 2>(a, st);
-        default: return layer_launch<NC, 4, 4>(a, st);
+    switch (f.tiles * 2 + f.steps) {
+        case 2 + 1: return layer_launch<NC, 1, 1>(a, st);
+        case 2 + 2: return layer_launch<NC, 1, 2>(a, st);
+        case 4 + 1: return layer_launch<NC, 2, 1>(a, st);
+        case 4 + 2: return layer_launch<NC, 2, 2>(a, st);
+        case 8 + 1: return layer_launch<NC, 4, 1>(a, st);
+        default: return layer_launch<NC, 4, 2>(a, st);
     }
 }
 
@@ -505,7 +493,7 @@ int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
 // product), which brings both to the square root of their product.  After that A has one scale
 // per row (o, s') and B one per input channel, each common to the 8 columns of a step: neither the
 // size of a right-hand side nor that of a channel costs bits.
-// Both operands keep 24 bits (split_rest): the first pieces' products add up exactly (K <= 64), the
+// Both operands keep 24 bits as the layer's: the first pieces' products add up exactly (K <= 64), the
 // other five go to a second accumulator.  A step's products (6 NC MMAs per tile, one rounding)
 // are added to FP64 sums in shared memory; warps, blocks and chunks are summed in a fixed order.
 constexpr int kGradWarps = 8;

@@ -100,3 +100,24 @@ def test_gradient_of_unequal_spins(oracle_lib, L, nc, m, layers, ch):
     _, ref_grads = oracle_lib.precond_loss_grad(b, ws, g, L, kappa, -1.0)
     for s in range(4):
         assert rel_err(grads[0][..., s], ref_grads[0][..., s]) <= 4e-6
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", SHAPES + [((2, 2, 2, 2), 3, 3, 1, 1)])
+@pytest.mark.parametrize("octaves", [0, 10, 20])
+def test_identity_network_keeps_24_bits(L, nc, m, layers, ch, octaves):
+    """Entries down to 2^-21 of a column's largest pass the identity path within a unit of the last
+    of 24 bits of themselves in every layer."""
+    rng = np.random.default_rng(600 + ch + m)
+    g, _, b = _case(L, nc, m, layers, ch, 600 + ch + m, 1.0)
+    part = lambda: rng.choice([-1, 1], b.shape) * rng.uniform(0.5, 1, b.shape) * 2.0 ** -rng.uniform(0, octaves, b.shape)
+    b = (part() + 1j * part()).astype(np.complex64).astype(np.complex128)
+    P = LearnedPreconditioner(L, nc, m, layers, ch, t_boundary=-1.0)
+    P.set_weights(identity_weights(layers, ch))
+    P.set_gauge(to_dev(g))
+    out = to_dev(np.zeros_like(b), q.SINGLE)
+    P.apply(out, to_dev(b, q.SINGLE), precision=q.SINGLE)
+    q.lib().qcuDeviceSynchronize()
+    d = from_dev(out) - b
+    P.close()
+    assert np.all(np.abs(d.real) <= layers * 2.0 ** -23 * np.abs(b.real))
+    assert np.all(np.abs(d.imag) <= layers * 2.0 ** -23 * np.abs(b.imag))
