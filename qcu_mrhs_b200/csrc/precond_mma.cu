@@ -6,8 +6,10 @@
 // neighbour spinors).  The link acts on the product's colours, in FP32.
 //
 // FP32 products on the 16-bit MMA (mma.sync m16n8k16, FP32 accumulation): operands are scaled
-// by powers of two so that their largest entries sit at 2^14 (the weights per layer, every
-// column of a field per path) and split into FP16 pieces.
+// by powers of two so that their largest entries sit at 2^14 and split into FP16 pieces.  On every
+// path the weights have a scale per row (o, s') and per input channel, w_oi / (q_o p_i) against
+// p_i x_i, and the field one per column of p_i x_i: neither the size of a channel, between which a
+// linear network is free to shift factors, nor that of a right-hand side costs bits.
 //   first pieces  w0, x0: the values rounded to multiples of 2^6, so 9 bits of the largest entry.
 //                 Products of two of them are multiples of 2^12 up to 2^30, and 64 of them (the
 //                 largest K that one accumulator sees) add up within 24 bits: exact.
@@ -100,8 +102,9 @@ __device__ __forceinline__ float scale_to_half(float m, float* inv) {
 }
 
 // ---- weights ----
-// A fragments of one layer: [path][row tile][K step][piece][lane] uint4, then at the end the
-// inverse of the layer's scale.  adj: of the adjoint layer, W'[i][o][-k] = W[o][i][k]^dag.
+// A fragments of one layer: [path][row tile][K step][piece][lane] uint4, then for
+// every path the input channels' factors p_i and the rows' inverse scales.  adj: of the adjoint
+// layer, W'[i][o][-k] = W[o][i][k]^dag.
 struct FragShape {
     int mt, ks;        // row tiles (2 output channels each) and K steps (2 input channels), padded
     int tiles, steps;  // per block and per channel chunk
@@ -117,11 +120,14 @@ FragShape frag_shape(int cin, int cout) {
     return s;
 }
 
+__host__ __device__ inline int frag_channels(int ks) { return 2 * ks; }
+__host__ __device__ inline int frag_rows(int mt) { return 8 * mt; }
+
 struct PrepLayer {
     const float2* w;
     uint4* frag;
-    float* inv;
-    int cin, cout;     // of the layer that the fragments compute
+    float *chan, *row;   // [path][2 ks] factors of the input channels, [path][8 mt] inverse row scales
+    int cin, cout;       // of the layer that the fragments compute
     int mt, ks;
 };
 struct PrepArgs {
@@ -131,46 +137,83 @@ struct PrepArgs {
 
 __device__ __forceinline__ int opposite_path(int k) { return k == 0 ? 0 : (((k - 1) & 1) ? k - 1 : k + 1); }
 
+__device__ __forceinline__ float finite_abs(float v) { return fabsf(v) <= 3.4028235e38f ? fabsf(v) : 0.f; }
+
+// power of two at or below m (of the smallest normal number for m below it), and its inverse
+__device__ __forceinline__ float power_of(float m, float* inv) {
+    const int e = min(max((int)(__float_as_uint(m) >> 23), 1), 253);
+    *inv = __uint_as_float((uint32_t)(254 - e) << 23);
+    return __uint_as_float((uint32_t)e << 23);
+}
+
+// One block per (layer, path).
 __global__ void ptc_prepare_kernel(PrepArgs a) {
     const PrepLayer L = a.l[blockIdx.x];
-    const int n = L.cin * L.cout * kPaths * 16;
-    __shared__ float wmax[32];
-    float mx = 0.f;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) mx = fmaxf(mx, fmaxf(fabsf(L.w[e].x), fabsf(L.w[e].y)));
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
+    const int k = blockIdx.y;
+    // maxima as bit patterns (ordered as the numbers): rows, channels of w / q, rows of w / (q p).
+    // The rows first, so that p_i is at most 1 and p_i x_i does not overflow.
+    __shared__ unsigned qmax[64], cmax[16], rmax[64];
+    // entry (o, s'), (i, s) of the path's matrix
+    auto weight = [&](int o, int sp, int i, int t) {
+        if (!a.adj) return L.w[((int64_t)(o * L.cin + i) * kPaths + k) * 16 + sp * 4 + t];
+        // stored W[o' = i][i' = o][opposite k][s' = t][s = sp]
+        const float2 v = L.w[((int64_t)(i * L.cout + o) * kPaths + opposite_path(k)) * 16 + t * 4 + sp];
+        return make_float2(v.x, -v.y);
+    };
+    auto inverse = [](unsigned m) {
+        float inv;
+        power_of(__uint_as_float(m), &inv);
+        return inv;
+    };
+    const int n = L.cin * L.cout * 16;
+    for (int e = threadIdx.x; e < 64; e += blockDim.x) {
+        qmax[e] = rmax[e] = 0u;
+        if (e < 16) cmax[e] = 0u;
+    }
     __syncthreads();
-    mx = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) mx = fmaxf(mx, wmax[i]);
-    float inv;
-    const float sc = scale_to_half(mx, &inv);
-    if (threadIdx.x == 0) *L.inv = inv;
-    const int total = kPaths * L.mt * L.ks * 32;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-        const int lane = e & 31, j = (e >> 5) % L.ks, q = (e >> 5) / L.ks;
-        const int mt = q % L.mt, k = q / L.mt;
+#pragma unroll 1
+    for (int pass = 0; pass < 3; ++pass) {
+        for (int e = threadIdx.x; e < n; e += blockDim.x) {
+            const int i = (e >> 4) % L.cin, o = (e >> 4) / L.cin, sp = (e >> 2) & 3, r = 4 * o + sp;
+            const float2 v = weight(o, sp, i, e & 3);
+            // an infinity decides over no other entry
+            float mx = fmaxf(finite_abs(v.x), finite_abs(v.y));
+            if (pass > 0) mx *= inverse(qmax[r]);
+            if (pass > 1) mx *= inverse(cmax[i]);
+            atomicMax(pass == 0 ? &qmax[r] : (pass == 1 ? &cmax[i] : &rmax[r]), __float_as_uint(mx));
+        }
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < frag_channels(L.ks); i += blockDim.x) {
+        float inv;
+        L.chan[k * frag_channels(L.ks) + i] = power_of(__uint_as_float(cmax[i]), &inv);
+    }
+    for (int r = threadIdx.x; r < frag_rows(L.mt); r += blockDim.x) {
+        float inv, qinv;
+        scale_to_half(__uint_as_float(rmax[r]), &inv);
+        L.row[k * frag_rows(L.mt) + r] = inv * power_of(__uint_as_float(qmax[r]), &qinv);
+    }
+    for (int e = threadIdx.x; e < L.mt * L.ks * 32; e += blockDim.x) {
+        const int lane = e & 31, j = (e >> 5) % L.ks, mt = (e >> 5) / L.ks;
         const int g = lane >> 2, t = lane & 3;
         const int o = 2 * mt + (g >> 2), sp = g & 3;
+        float inv;
+        const float sc = scale_to_half(__uint_as_float(rmax[4 * o + sp]), &inv);
         uint32_t w0[4], w1[4], w2[4];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             const int i = 2 * j + c;
             float2 v = make_float2(0.f, 0.f);
             if (o < L.cout && i < L.cin) {
-                if (a.adj) {   // stored W[o' = i][i' = o][opposite k][s' = t][s = sp]
-                    v = L.w[((int64_t)(i * L.cout + o) * kPaths + opposite_path(k)) * 16 + t * 4 + sp];
-                    v.y = -v.y;
-                } else {
-                    v = L.w[((int64_t)(o * L.cin + i) * kPaths + k) * 16 + sp * 4 + t];
-                }
+                v = weight(o, sp, i, t);
+                const float qi = inverse(qmax[4 * o + sp]), pi = inverse(cmax[i]);
+                v.x = v.x * qi * pi * sc;   // in this order: 0 <= |w| / q < 2, w / (q p) < 2
+                v.y = v.y * qi * pi * sc;
             }
-            v.x *= sc;
-            v.y *= sc;
             split_rest(make_float2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
             split_rest(make_float2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
         }
-        uint4* f = L.frag + (int64_t)(e >> 5) * kStepVecs + lane;
+        uint4* f = L.frag + (int64_t)(((k * L.mt + mt) * L.ks + j)) * kStepVecs + lane;
         f[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
         f[32] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
         f[64] = make_uint4(w2[0], w2[1], w2[2], w2[3]);
@@ -182,7 +225,7 @@ struct LayerArgs {
     float2* out;
     const float2* in;
     const uint4* frag;
-    const float* inv;
+    const float *chan, *row;
     const float2* gauge;
     Geom g;
     int m, cin, cout, mt, ks;
@@ -250,6 +293,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -278,8 +326,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
         const int k = e / per_path, r = e - k * per_path;
         sw[e] = a.frag[(int64_t)(k * a.mt + mt0) * a.ks * kStepVecs + r];
     }
+    const int nch = frag_channels(a.ks);
+    float* const chan = reinterpret_cast<float*>(sw + kPaths * per_path);   // [path][2 ks]
+    float* const row = chan + kPaths * nch;                                 // [path][8 MT]
+    for (int e = threadIdx.x; e < kPaths * nch; e += blockDim.x) chan[e] = a.chan[e];
+    for (int e = threadIdx.x; e < kPaths * frag_rows(MT); e += blockDim.x)
+        row[e] = a.row[(e / frag_rows(MT)) * frag_rows(a.mt) + frag_rows(mt0) + e % frag_rows(MT)];
     __syncthreads();
-    const float winv = *a.inv;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int m = a.m;
     const uint32_t um = (uint32_t)m;
@@ -331,15 +384,20 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
         for (int k = 0, j0 = 0; k < kPaths;) {
             float mx = 0.f;
 #pragma unroll
-            for (int i = 0; i < 2 * KS; ++i)
+            for (int i = 0; i < 2 * KS; ++i) {
+                const float pc = chan[k * nch + 2 * j0 + i];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) mx = fmaxf(mx, fmaxf(fabsf(x[i][c].x), fabsf(x[i][c].y)));
+                for (int c = 0; c < NC; ++c) {
+                    x[i][c].x *= pc;
+                    x[i][c].y *= pc;
+                    mx = fmaxf(mx, fmaxf(fabsf(x[i][c].x), fabsf(x[i][c].y)));
+                }
+            }
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             float inv;
             const float sc = scale_to_half(mx, &inv);
-            // scale, link and boundary of this lane's D columns 2t and 2t + 1; the scale goes into
-            // the link
+            // scale, link and boundary of this lane's D columns 2t and 2t + 1
             float dinv[2];
             f32x2 ur[NC][NC], ui[NC][NC];
 #pragma unroll
@@ -348,7 +406,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
                 const bool fwd = (k & 1) != 0;
                 const int w0 = __shfl_sync(0xffffffffu, (int)wrap, 8 * t), w1 = __shfl_sync(0xffffffffu, (int)wrap, 8 * t + 4);
                 const uint32_t l1 = __shfl_sync(0xffffffffu, link, 8 * t + 4);
-                const float s0 = w0 ? a.t_sign * dinv[0] : dinv[0], s1 = w1 ? a.t_sign * dinv[1] : dinv[1];
+                const float s0 = w0 ? a.t_sign : 1.f, s1 = w1 ? a.t_sign : 1.f;
                 const float2* U = a.gauge + (int64_t)l1 * (NC * NC);
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
@@ -410,16 +468,17 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
                         }
                     }
                     const f32x2 kr = pack2(kRest, kRest);
+                    const float rinv = row[k0 * frag_rows(MT) + 8 * q + g];
+                    const f32x2 back = pack2(rinv * dinv[0], rinv * dinv[1]);
 #pragma unroll
                     for (int c = 0; c < CG; ++c) {
-                        const f32x2 dr = fma2(pack2(d2[c][0], d2[c][1]), kr, pack2(d1[c][0], d1[c][1]));
-                        const f32x2 di = fma2(pack2(d2[c][2], d2[c][3]), kr, pack2(d1[c][2], d1[c][3]));
+                        const f32x2 dr = mul2(fma2(pack2(d2[c][0], d2[c][1]), kr, pack2(d1[c][0], d1[c][1])), back);
+                        const f32x2 di = mul2(fma2(pack2(d2[c][2], d2[c][3]), kr, pack2(d1[c][2], d1[c][3])), back);
                         if (k0 == 0) {
-                            const f32x2 s = pack2(dinv[0], dinv[1]);
-                            re[q][c0 + c] = fma2(s, dr, re[q][c0 + c]);
-                            im[q][c0 + c] = fma2(s, di, im[q][c0 + c]);
+                            re[q][c0 + c] = add2(re[q][c0 + c], dr);
+                            im[q][c0 + c] = add2(im[q][c0 + c], di);
                         } else {
-                            const f32x2 nd = fma2(di, pack2(-1.f, -1.f), 0ull);
+                            const f32x2 nd = mul2(di, pack2(-1.f, -1.f));
 #pragma unroll
                             for (int r = 0; r < NC; ++r) {
                                 re[q][r] = fma2(ur[r][c0 + c], dr, re[q][r]);
@@ -447,9 +506,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
                     const float2 r2 = unpack2(re[q][c]), i2 = unpack2(im[q][c]);
                     if (!odd)   // both columns: adjacent RHS of one site
                         *reinterpret_cast<float4*>(dst + c * m) =
-                            make_float4(r2.x * winv, i2.x * winv, r2.y * winv, i2.y * winv);
+                            make_float4(r2.x, i2.x, r2.y, i2.y);
                     else
-                        dst[c * m] = make_float2((b ? r2.y : r2.x) * winv, (b ? i2.y : i2.x) * winv);
+                        dst[c * m] = b ? make_float2(r2.y, i2.y) : make_float2(r2.x, i2.x);
                 }
             }
         }
@@ -459,7 +518,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
 template <int NC, int MT, int KS>
 int layer_launch(const LayerArgs& a, cudaStream_t st) {
     auto k = ptc_mma_kernel<NC, MT, KS>;
-    const size_t smem = (size_t)kPaths * MT * a.ks * kStepBytes;
+    const size_t smem = (size_t)kPaths * (MT * a.ks * kStepBytes + (frag_channels(a.ks) + frag_rows(MT)) * sizeof(float));
     if (int rc = smem_optin(reinterpret_cast<const void*>(k), smem)) return rc;
     const int ny = a.mt / MT;
     const int64_t tiles = (2 * a.g.vh * a.m + 7) / 8, want = (tiles + kMmaThreads / 32 - 1) / (kMmaThreads / 32);
@@ -516,7 +575,6 @@ __device__ __forceinline__ float balance(float h, float x, float* inv) {
     *inv = __uint_as_float((uint32_t)(127 - c) << 23);
     return __uint_as_float((uint32_t)(127 + c) << 23);
 }
-__device__ __forceinline__ float finite_abs(float v) { return fabsf(v) <= 3.4028235e38f ? fabsf(v) : 0.f; }
 
 // maximum over the 8 lanes of one column pair (t), and over the 4 lanes of one row (g)
 __device__ __forceinline__ float column_max(float v) {
@@ -816,8 +874,24 @@ int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* 
 
 size_t ptc_frag_bytes(int cin, int cout) {
     const FragShape f = frag_shape(cin, cout);
-    return (size_t)kPaths * f.mt * f.ks * kStepBytes + 16;
+    const size_t b = (size_t)kPaths * (f.mt * f.ks * kStepBytes + (frag_channels(f.ks) + frag_rows(f.mt)) * sizeof(float));
+    return (b + 15) & ~(size_t)15;
 }
+
+namespace {
+// the parts of a layer's fragments
+struct FragParts {
+    uint4* frag;
+    float *chan, *row;
+};
+FragParts frag_parts(void* base, const FragShape& f) {
+    FragParts p;
+    p.frag = static_cast<uint4*>(base);
+    p.chan = reinterpret_cast<float*>(p.frag + (size_t)kPaths * f.mt * f.ks * kStepVecs);
+    p.row = p.chan + kPaths * frag_channels(f.ks);
+    return p;
+}
+}  // namespace
 
 int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
                 cudaStream_t st) {
@@ -826,11 +900,10 @@ int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const
     for (int l = 0; l < layers; ++l) {
         const int ci = adj ? cout[l] : cin[l], co = adj ? cin[l] : cout[l];
         const FragShape f = frag_shape(ci, co);
-        char* base = static_cast<char*>(frag[l]);
-        a.l[l] = PrepLayer{w[l], reinterpret_cast<uint4*>(base),
-                           reinterpret_cast<float*>(base + (size_t)kPaths * f.mt * f.ks * kStepBytes), ci, co, f.mt, f.ks};
+        const FragParts p = frag_parts(frag[l], f);
+        a.l[l] = PrepLayer{w[l], p.frag, p.chan, p.row, ci, co, f.mt, f.ks};
     }
-    ptc_prepare_kernel<<<layers, 256, 0, st>>>(a);
+    ptc_prepare_kernel<<<dim3(layers, kPaths), 256, 0, st>>>(a);
     QCUB_CHECK_LAUNCH();
     return QCU_SUCCESS;
 }
@@ -838,10 +911,8 @@ int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const
 int ptc_layer(int nc, float2* out, const float2* in, const void* frag, const float2* gauge, const Geom& g, int m,
               int cin, int cout, float t_sign, const int* done, cudaStream_t st) {
     const FragShape f = frag_shape(cin, cout);
-    const char* base = static_cast<const char*>(frag);
-    const LayerArgs a{out, in, reinterpret_cast<const uint4*>(base),
-                      reinterpret_cast<const float*>(base + (size_t)kPaths * f.mt * f.ks * kStepBytes), gauge, g, m, cin, cout,
-                      f.mt, f.ks, t_sign, done};
+    const FragParts p = frag_parts(const_cast<void*>(frag), f);
+    const LayerArgs a{out, in, p.frag, p.chan, p.row, gauge, g, m, cin, cout, f.mt, f.ks, t_sign, done};
     switch (nc) {
         case 2: return layer_nc<2>(a, f, st);
         case 3: return layer_nc<3>(a, f, st);

@@ -121,3 +121,72 @@ def test_identity_network_keeps_24_bits(L, nc, m, layers, ch, octaves):
     P.close()
     assert np.all(np.abs(d.real) <= layers * 2.0 ** -23 * np.abs(b.real))
     assert np.all(np.abs(d.imag) <= layers * 2.0 ** -23 * np.abs(b.imag))
+
+
+def _unequal_channels(ws, factor, balanced):
+    """Channel o of every layer between two others times factor^(o mod 3), its weights in the next
+    layer times the inverse (balanced: the network is the same) or as they are."""
+    ws = [w.copy() for w in ws]
+    for l in range(len(ws) - 1):
+        d = factor ** (np.arange(ws[l].shape[0]) % 3)
+        ws[l] *= d[:, None, None, None, None]
+        if balanced:
+            ws[l + 1] /= d[None, :, None, None, None]
+    return [w.astype(np.complex64).astype(np.complex128) for w in ws]
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", [s for s in SHAPES if s[4] > 1])
+@pytest.mark.parametrize("factor,balanced", [(1e-2, True), (1e-2, False), (1e-3, True)])
+def test_gradient_of_unequal_channels(oracle_lib, L, nc, m, layers, ch, factor, balanced):
+    """Every (output, input channel) block of the gradient to the tolerance of the whole."""
+    kappa = 0.12
+    g, ws, b = _case(L, nc, m, layers, ch, 400 + ch + m, 1.0)
+    ws = _unequal_channels(ws, factor, balanced)
+    _, grads = _loss_grad(L, nc, m, layers, ch, g, ws, b, kappa)
+    _, ref_grads = oracle_lib.precond_loss_grad(b, ws, g, L, kappa, -1.0)
+    for gg, rg in zip(grads, ref_grads):
+        for o in range(rg.shape[0]):
+            for i in range(rg.shape[1]):
+                assert rel_err(gg[o, i], rg[o, i]) <= 4e-6
+
+
+def _apply(L, nc, m, layers, ch, g, ws, b):
+    P = LearnedPreconditioner(L, nc, m, layers, ch, t_boundary=-1.0)
+    P.set_weights(ws)
+    P.set_gauge(to_dev(g))
+    out = to_dev(np.zeros_like(b), q.SINGLE)
+    P.apply(out, to_dev(b, q.SINGLE), precision=q.SINGLE)
+    q.lib().qcuDeviceSynchronize()
+    P.close()
+    return from_dev(out)
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", [s for s in SHAPES if s[4] > 1])
+@pytest.mark.parametrize("factor", [1e-2, 1e-5, 1e-9])
+def test_apply_with_unequal_channels(oracle_lib, L, nc, m, layers, ch, factor):
+    """Factors shifted between a channel and its weights leave the network and its errors alone."""
+    g, ws, b = _case(L, nc, m, layers, ch, 700 + ch + m, 1.0)
+    ws = _unequal_channels(ws, factor, True)
+    ref = oracle_lib.precond_apply(b, ws, g, L, -1.0)
+    assert rel_err(_apply(L, nc, m, layers, ch, g, ws, b), ref) <= 2e-6
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", [s for s in SHAPES if s[4] > 1])
+def test_apply_of_a_small_row(oracle_lib, L, nc, m, layers, ch):
+    """An output channel of tiny weights beside ordinary ones, and nothing else of the layer in the
+    output."""
+    g, ws, b = _case(L, nc, m, layers, ch, 800 + ch + m, 1.0)
+    ws[0][1] *= 1e-10
+    ws[1][:, [i for i in range(ch) if i != 1]] = 0.0
+    ws = [w.astype(np.complex64).astype(np.complex128) for w in ws]
+    ref = oracle_lib.precond_apply(b, ws, g, L, -1.0)
+    assert rel_err(_apply(L, nc, m, layers, ch, g, ws, b), ref) <= 2e-6
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", SHAPES)
+@pytest.mark.parametrize("size", [1e34, 1e-30])
+def test_apply_keeps_the_range_of_fp32(oracle_lib, L, nc, m, layers, ch, size):
+    g, ws, b = _case(L, nc, m, layers, ch, 900 + ch + m, 1.0)
+    b = (b * size).astype(np.complex64).astype(np.complex128)
+    ref = oracle_lib.precond_apply(b, ws, g, L, -1.0)
+    assert rel_err(_apply(L, nc, m, layers, ch, g, ws, b), ref) <= 2e-6
