@@ -340,7 +340,8 @@ int Precond::loss_grad(const float2* b, double kappa, double* loss, cudaStream_t
     for (int l = layers - 1; l >= 0; --l) {
         const float2* gout = static_cast<const float2*>(gbuf[cur].ptr);
         if ((rc = ptc_grad(nc, static_cast<double2*>(gw.ptr) + woff[l], gpart.ptr, gout,
-                           fields + (int64_t)act_offset(l) * fl, gp, g, m, cin[l], cout[l], (float)t_sign, st)))
+                           fields + (int64_t)act_offset(l) * fl, gp, dn + kMaxRhs, g, m, cin[l], cout[l],
+                           (float)t_sign, st)))
             return rc;
         if (l == 0) break;
         if ((rc = ptc_layer(nc, static_cast<float2*>(gbuf[1 - cur].ptr), gout,

@@ -64,10 +64,10 @@ int ptc_layer(int nc, float2* out, const float2* in, const void* frag, const flo
               int cin, int cout, float t_sign, const int* done, cudaStream_t st);
 
 // weight gradient gw[o][i][k][s'][s] = sum gout_o[s'] conj((T_k in_i)[s]); part: scratch of
-// ptc_grad_bytes
+// ptc_grad_bytes; bnorm: sizes of the right-hand sides that in goes as and gout inversely
 size_t ptc_grad_bytes(int cin, int cout);
-int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge, const Geom& g,
-             int m, int cin, int cout, float t_sign, cudaStream_t st);
+int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge,
+             const double* bnorm, const Geom& g, int m, int cin, int cout, float t_sign, cudaStream_t st);
 
 // Right-preconditioned BiCGStab on the full system M x = b (solver.cu).
 int solve_precond(Context& c, Precond* P, void* x, const void* b, int max_iter, double tol);

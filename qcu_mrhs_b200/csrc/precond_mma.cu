@@ -150,9 +150,9 @@ __device__ __forceinline__ float power_of(float m, float* inv) {
 __global__ void ptc_prepare_kernel(PrepArgs a) {
     const PrepLayer L = a.l[blockIdx.x];
     const int k = blockIdx.y;
-    // maxima as bit patterns (ordered as the numbers): rows, channels of w / q, rows of w / (q p).
-    // The rows first, so that p_i is at most 1 and p_i x_i does not overflow.
+    // maxima as bit patterns (ordered as the numbers): rows, channels of w / q, rows of w / (q p)
     __shared__ unsigned qmax[64], cmax[16], rmax[64];
+    __shared__ int shift;
     // entry (o, s'), (i, s) of the path's matrix
     auto weight = [&](int o, int sp, int i, int t) {
         if (!a.adj) return L.w[((int64_t)(o * L.cin + i) * kPaths + k) * 16 + sp * 4 + t];
@@ -160,11 +160,7 @@ __global__ void ptc_prepare_kernel(PrepArgs a) {
         const float2 v = L.w[((int64_t)(i * L.cout + o) * kPaths + opposite_path(k)) * 16 + t * 4 + sp];
         return make_float2(v.x, -v.y);
     };
-    auto inverse = [](unsigned m) {
-        float inv;
-        power_of(__uint_as_float(m), &inv);
-        return inv;
-    };
+    auto exponent = [](unsigned m) { return max((int)(m >> 23), 1) - 127; };
     const int n = L.cin * L.cout * 16;
     for (int e = threadIdx.x; e < 64; e += blockDim.x) {
         qmax[e] = rmax[e] = 0u;
@@ -178,20 +174,26 @@ __global__ void ptc_prepare_kernel(PrepArgs a) {
             const float2 v = weight(o, sp, i, e & 3);
             // an infinity decides over no other entry
             float mx = fmaxf(finite_abs(v.x), finite_abs(v.y));
-            if (pass > 0) mx *= inverse(qmax[r]);
-            if (pass > 1) mx *= inverse(cmax[i]);
+            if (pass > 0) mx = scalbnf(mx, -exponent(qmax[r]) - (pass > 1 ? exponent(cmax[i]) : 0));
             atomicMax(pass == 0 ? &qmax[r] : (pass == 1 ? &cmax[i] : &rmax[r]), __float_as_uint(mx));
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < frag_channels(L.ks); i += blockDim.x) {
-        float inv;
-        L.chan[k * frag_channels(L.ks) + i] = power_of(__uint_as_float(cmax[i]), &inv);
+    // the channels' factors lie between 2^-126 and 2 so far; their middle goes to 1, so that p_i x_i
+    // leaves FP32's range on either side only where the channels' sizes differ by as much
+    if (threadIdx.x == 0) {
+        int lo = 0;
+        for (int i = 0; i < L.cin; ++i)
+            if (cmax[i] != 0u) lo = min(lo, exponent(cmax[i]));
+        shift = -lo / 2;
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < frag_channels(L.ks); i += blockDim.x)
+        L.chan[k * frag_channels(L.ks) + i] = scalbnf(1.f, exponent(cmax[i]) + (cmax[i] != 0u ? shift : 0));
     for (int r = threadIdx.x; r < frag_rows(L.mt); r += blockDim.x) {
-        float inv, qinv;
+        float inv;
         scale_to_half(__uint_as_float(rmax[r]), &inv);
-        L.row[k * frag_rows(L.mt) + r] = inv * power_of(__uint_as_float(qmax[r]), &qinv);
+        L.row[k * frag_rows(L.mt) + r] = scalbnf(inv, exponent(qmax[r]) - shift);
     }
     for (int e = threadIdx.x; e < L.mt * L.ks * 32; e += blockDim.x) {
         const int lane = e & 31, j = (e >> 5) % L.ks, mt = (e >> 5) / L.ks;
@@ -206,9 +208,9 @@ __global__ void ptc_prepare_kernel(PrepArgs a) {
             float2 v = make_float2(0.f, 0.f);
             if (o < L.cout && i < L.cin) {
                 v = weight(o, sp, i, t);
-                const float qi = inverse(qmax[4 * o + sp]), pi = inverse(cmax[i]);
-                v.x = v.x * qi * pi * sc;   // in this order: 0 <= |w| / q < 2, w / (q p) < 2
-                v.y = v.y * qi * pi * sc;
+                const int e2 = -exponent(qmax[4 * o + sp]) - exponent(cmax[i]);
+                v.x = scalbnf(v.x, e2) * sc;
+                v.y = scalbnf(v.y, e2) * sc;
             }
             split_rest(make_float2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
             split_rest(make_float2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
@@ -547,11 +549,11 @@ int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
 // transported gradient; B: columns (i, s, re/im), the pair (v.re, v.im) for the real part and
 // (-v.im, v.re) for the imaginary part, so a lane's D registers are whole complex numbers.
 // A column is a (site, RHS) pair, and the operands' sizes run in opposite directions: the loss
-// divides by ||b_j||^2, so g goes as 1 / ||b_j|| where in goes as ||b_j||.  Every column therefore
-// takes a power of two p from its largest entries, g p and in / p (exact, and gone from the
-// product), which brings both to the square root of their product.  After that A has one scale
-// per row (o, s') and B one per input channel, each common to the 8 columns of a step: neither the
-// size of a right-hand side nor that of a channel costs bits.
+// divides by ||b_j||^2, so g goes as 1 / ||b_j|| where in goes as ||b_j|| (the layers are linear).  The
+// columns of right-hand side j are therefore taken as g p and in / p with the power of two p at
+// ||b_j||: exact, and gone from the product.  After that A has one scale per row (o, s') and B one
+// per input channel, each common to the 8 columns of a step: neither the size of a right-hand side
+// nor that of a channel costs bits, and a channel that overflows does so alone.
 // Both operands keep 24 bits as the layer's: the first pieces' products add up exactly (K <= 64), the
 // other five go to a second accumulator.  A step's products (6 NC MMAs per tile, one rounding)
 // are added to FP64 sums in shared memory; warps, blocks and chunks are summed in a fixed order.
@@ -563,25 +565,13 @@ struct GradArgs {
     const float2* gout;
     const float2* in;
     const float2* gauge;
+    const double* bnorm;   // ||b_j||
     Geom g;
     int m, cin, cout;
     float t_sign;
 };
 
-// power of two nearest to sqrt(x / h) for a column's largest entries h and x, and its inverse
-__device__ __forceinline__ float balance(float h, float x, float* inv) {
-    const int d = ((int)(__float_as_uint(x) >> 23) - (int)(__float_as_uint(h) >> 23)) >> 1;
-    const int c = min(max(d, -126), 126);
-    *inv = __uint_as_float((uint32_t)(127 - c) << 23);
-    return __uint_as_float((uint32_t)(127 + c) << 23);
-}
-
-// maximum over the 8 lanes of one column pair (t), and over the 4 lanes of one row (g)
-__device__ __forceinline__ float column_max(float v) {
-#pragma unroll
-    for (int off = 16; off >= 4; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
-    return v;
-}
+// maximum over the 4 lanes of a row (g)
 __device__ __forceinline__ float row_max(float v) {
     v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
     return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
@@ -596,6 +586,13 @@ __device__ __forceinline__ float warp_max(float v) {
 template <int NC, int MT, int CI>
 __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const GradArgs a) {
     extern __shared__ double sacc[];   // [warp][MT CI 4][lane]
+    __shared__ float2 sizes[kMaxRhs];  // the right-hand sides' powers of two and their inverses
+    if (threadIdx.x < a.m) {
+        float inv;
+        const float p = power_of((float)a.bnorm[threadIdx.x], &inv);
+        sizes[threadIdx.x] = make_float2(p, inv);
+    }
+    __syncthreads();
     constexpr int NA = MT * CI * 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int k = blockIdx.y, ni = (a.cin + CI - 1) / CI;
@@ -672,42 +669,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                 xs[i][c][1] = __ldg(v1 + fo + c * m);
             }
         }
-        // the columns' powers of two
-        float pc[2], pi[2];
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            float hm = 0.f, xm = 0.f;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-#pragma unroll
-                for (int q = 0; q < MT; ++q)
-#pragma unroll
-                    for (int w = 0; w < 2; ++w)
-                        hm = fmaxf(hm, fmaxf(fabsf(h[q][2 * b + w][c].x), fabsf(h[q][2 * b + w][c].y)));
-#pragma unroll
-                for (int i = 0; i < CI; ++i) xm = fmaxf(xm, fmaxf(fabsf(xs[i][c][b].x), fabsf(xs[i][c][b].y)));
-            }
-            hm = column_max(hm);
-            xm = column_max(xm);
-            // an infinity (of one channel) does not decide over the other channels' bits
-            if (__any_sync(0xffffffffu, fmaxf(hm, xm) > 3.4028235e38f)) {
-                hm = xm = 0.f;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-#pragma unroll
-                    for (int q = 0; q < MT; ++q)
-#pragma unroll
-                        for (int w = 0; w < 2; ++w)
-                            hm = fmaxf(hm, fmaxf(finite_abs(h[q][2 * b + w][c].x), finite_abs(h[q][2 * b + w][c].y)));
-#pragma unroll
-                    for (int i = 0; i < CI; ++i)
-                        xm = fmaxf(xm, fmaxf(finite_abs(xs[i][c][b].x), finite_abs(xs[i][c][b].y)));
-                }
-                hm = column_max(hm);
-                xm = column_max(xm);
-            }
-            pc[b] = balance(hm, xm, &pi[b]);
-        }
+        const float2 size[2] = {sizes[rr[0]], sizes[rr[1]]};
         float ainv[MT][2];
         uint4 a0[MT][NC], a1[MT][NC], a2[MT][NC];
 #pragma unroll
@@ -721,8 +683,8 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         float2& v = h[q][2 * b + w][c];
-                        v.x *= pc[b];
-                        v.y *= pc[b];
+                        v.x *= size[b].x;
+                        v.y *= size[b].x;
                         mx = fmaxf(mx, fmaxf(fabsf(v.x), fabsf(v.y)));
                     }
                 asc[w] = scale_to_half(row_max(mx), &ainv[q][w]);
@@ -746,8 +708,8 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
             for (int c = 0; c < NC; ++c)
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    x[c][b].x *= pi[b];
-                    x[c][b].y *= pi[b];
+                    x[c][b].x *= size[b].y;
+                    x[c][b].y *= size[b].y;
                     bx = fmaxf(bx, fmaxf(fabsf(x[c][b].x), fabsf(x[c][b].y)));
                 }
             float binv;
@@ -860,10 +822,10 @@ size_t ptc_grad_bytes(int cin, int cout) {
     return (size_t)kGradChunks * kPaths * s.nz * s.mt * s.ci * 128 * sizeof(double);
 }
 
-int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge, const Geom& g,
-             int m, int cin, int cout, float t_sign, cudaStream_t st) {
+int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge,
+             const double* bnorm, const Geom& g, int m, int cin, int cout, float t_sign, cudaStream_t st) {
     const GradShape s = grad_shape(cin, cout);
-    const GradArgs a{static_cast<double*>(part), gout, in, gauge, g, m, cin, cout, t_sign};
+    const GradArgs a{static_cast<double*>(part), gout, in, gauge, bnorm, g, m, cin, cout, t_sign};
     switch (nc) {
         case 2: return grad_nc<2>(a, s, gw, st);
         case 3: return grad_nc<3>(a, s, gw, st);

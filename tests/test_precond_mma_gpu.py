@@ -190,3 +190,20 @@ def test_apply_keeps_the_range_of_fp32(oracle_lib, L, nc, m, layers, ch, size):
     b = (b * size).astype(np.complex64).astype(np.complex128)
     ref = oracle_lib.precond_apply(b, ws, g, L, -1.0)
     assert rel_err(_apply(L, nc, m, layers, ch, g, ws, b), ref) <= 2e-6
+
+
+def test_gradient_beside_an_infinite_channel(oracle_lib):
+    """A channel whose output gradient overflows (its last weight is near FP32's largest number, its
+    own value is zero) leaves the other channels' gradients as they are."""
+    L, nc, m, ch, kappa = (4, 2, 2, 4), 3, 8, 4, 0.12
+    g, ws, b = _case(L, nc, m, 2, ch, 1000, 1.0)
+    ws[0][2] = 0.0
+    ws[1][0, 2] = 0.0
+    ws[1][0, 2, 0] = 3e38 * np.eye(4)
+    ws = [w.astype(np.complex64).astype(np.complex128) for w in ws]
+    _, grads = _loss_grad(L, nc, m, 2, ch, g, ws, b * 1e-5, kappa)
+    _, ref = oracle_lib.precond_loss_grad(b * 0.01, ws, g, L, kappa, -1.0)
+    assert not np.all(np.isfinite(grads[0][2]))
+    for o in (0, 1, 3):
+        assert rel_err(grads[0][o], ref[0][o]) <= 4e-6
+        assert rel_err(grads[1][0, o], ref[1][0, o]) <= 4e-6
