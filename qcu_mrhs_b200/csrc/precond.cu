@@ -237,8 +237,8 @@ int Precond::init(const int L[4], int n_color, int m_rhs, int n_layers, int chan
     for (int l = 0; l < layers; ++l) {
         foff.push_back(fb);
         faoff.push_back(fa);
-        fb += ptc_frag_bytes(cin[l], cout[l]);
-        fa += ptc_frag_bytes(cout[l], cin[l]);
+        fb += ptc_frag_bytes(nc, cin[l], cout[l]);
+        fa += ptc_frag_bytes(nc, cout[l], cin[l]);
         gb = std::max(gb, ptc_grad_bytes(cin[l], cout[l]));
     }
     int rc;
@@ -279,7 +279,7 @@ int Precond::prepare(bool adj, cudaStream_t st) {
         ws_[l] = static_cast<const float2*>(w.ptr) + woff[l];
         fs[l] = static_cast<char*>(adj ? fragadj.ptr : frag.ptr) + (adj ? faoff[l] : foff[l]);
     }
-    return ptc_prepare(ws_, fs, cin.data(), cout.data(), layers, adj, st);
+    return ptc_prepare(nc, ws_, fs, cin.data(), cout.data(), layers, adj, st);
 }
 
 void Precond::release() {
@@ -298,7 +298,8 @@ int Precond::apply(float2* out, const float2* in, const void* gauge32, cudaStrea
     const float2* src = in;
     for (int l = 0; l < layers; ++l) {
         float2* dst = (l == layers - 1) ? out : fields + (int64_t)act_offset(l + 1) * fl;
-        const int rc = ptc_layer(nc, dst, src, static_cast<const char*>(frag.ptr) + foff[l], gp, g, m, cin[l], cout[l],
+        const int rc = ptc_layer(nc, dst, src, static_cast<const float2*>(w.ptr) + woff[l], false,
+                                 static_cast<const char*>(frag.ptr) + foff[l], gp, g, m, cin[l], cout[l],
                                  (float)t_sign, done, st);
         if (rc) return rc;
         src = dst;
@@ -317,6 +318,7 @@ int Precond::loss_grad(const float2* b, double kappa, double* loss, cudaStream_t
     QCUB_CUDA_CHECK(cudaMemcpyAsync(fields, b, field_bytes(), cudaMemcpyDeviceToDevice, st));
     for (int l = 0; l < layers; ++l) {
         if ((rc = ptc_layer(nc, fields + (int64_t)act_offset(l + 1) * fl, fields + (int64_t)act_offset(l) * fl,
+                            static_cast<const float2*>(w.ptr) + woff[l], false,
                             static_cast<const char*>(frag.ptr) + foff[l], gp, g, m, cin[l], cout[l], (float)t_sign,
                             nullptr, st)))
             return rc;
@@ -345,6 +347,7 @@ int Precond::loss_grad(const float2* b, double kappa, double* loss, cudaStream_t
             return rc;
         if (l == 0) break;
         if ((rc = ptc_layer(nc, static_cast<float2*>(gbuf[1 - cur].ptr), gout,
+                            static_cast<const float2*>(w.ptr) + woff[l], true,
                             static_cast<const char*>(fragadj.ptr) + faoff[l], gp, g, m, cout[l], cin[l], (float)t_sign,
                             nullptr, st)))
             return rc;

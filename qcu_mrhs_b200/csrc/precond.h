@@ -54,14 +54,15 @@ struct Precond {
 
 // ---- layers (precond_mma.cu) ----
 // bytes of one layer's weight fragments
-size_t ptc_frag_bytes(int cin, int cout);
+size_t ptc_frag_bytes(int nc, int cin, int cout);
 // fragments of `layers` (<= 16) layers from their weights [cout][cin][9][4][4]; adj: of the
 // adjoint layers, from the same weights
-int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
+int ptc_prepare(int nc, const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
                 cudaStream_t st);
-// out_o = sum_i sum_k W[o][i][k] T_k in_i
-int ptc_layer(int nc, float2* out, const float2* in, const void* frag, const float2* gauge, const Geom& g, int m,
-              int cin, int cout, float t_sign, const int* done, cudaStream_t st);
+// out_o = sum_i sum_k W[o][i][k] T_k in_i; adj: the adjoint of the layer with weights w; frag: its
+// fragments
+int ptc_layer(int nc, float2* out, const float2* in, const float2* w, bool adj, const void* frag, const float2* gauge,
+              const Geom& g, int m, int cin, int cout, float t_sign, const int* done, cudaStream_t st);
 
 // weight gradient gw[o][i][k][s'][s] = sum gout_o[s'] conj((T_k in_i)[s]); part: scratch of
 // ptc_grad_bytes; bnorm: sizes of the right-hand sides that in goes as and gout inversely

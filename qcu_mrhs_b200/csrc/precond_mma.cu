@@ -63,30 +63,56 @@ __device__ __forceinline__ void mma16_zero(float (&d)[4], const uint4& a, uint32
 
 __device__ __forceinline__ uint32_t half_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 
-// v (below 2^15) rounded to a multiple of 2^6: adding 1.5 x 2^29 leaves no lower bits
-__device__ __forceinline__ float round_first(float v) {
-    constexpr float c = 1.5f * (float)(1 << 29);
-    return __fadd_rn(__fadd_rn(v, c), -c);
+// two FP32 numbers in one register pair and their packed arithmetic (same rounding as the
+// scalar instructions, half the issue slots)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
-// 2^9 on the rest's pieces, and what brings their products back
-constexpr float kRestUp = 512.f, kRest = 1.f / 512.f;
-__device__ __forceinline__ void split_float(float2 v, uint32_t& h, uint32_t& l) {   // v = h + l
-    const __half2 b = __float22half2_rn(v);
-    const float2 e = __half22float2(b);
+// Splits of a scaled pair (below 2^15).
+// v = h + l, both FP16
+__device__ __forceinline__ void split_float(f32x2 v, uint32_t& h, uint32_t& l) {
+    const __half2 b = __float22half2_rn(unpack2(v));
+    const float2 e = __half22float2(b), d = unpack2(fma2(pack2(e.x, e.y), pack2(-1.f, -1.f), v));
     h = half_bits(b);
-    l = half_bits(__floats2half2_rn(v.x - e.x, v.y - e.y));
+    l = half_bits(__float22half2_rn(d));
 }
-// first piece and 2^9 times the rest in two pieces of the pair v (scaled)
-__device__ __forceinline__ void split_rest(float2 v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    const float2 f = make_float2(round_first(v.x), round_first(v.y));
-    p0 = half_bits(__float22half2_rn(f));   // exact
-    split_float(make_float2((v.x - f.x) * kRestUp, (v.y - f.y) * kRestUp), p1, p2);
+// v rounded to a multiple of 2^6 (adding 1.5 x 2^29 leaves no lower bits), and 2^9 times the rest in
+// two pieces; kRest brings the rest's products back
+constexpr float kRestUp = 512.f, kRest = 1.f / 512.f;
+__device__ __forceinline__ void split_rest(f32x2 v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    constexpr float c = 1.5f * (float)(1 << 29);
+    const f32x2 f = add2(add2(v, pack2(c, c)), pack2(-c, -c));
+    p0 = half_bits(__float22half2_rn(unpack2(f)));   // exact
+    split_float(fma2(f, pack2(-kRestUp, -kRestUp), mul2(v, pack2(kRestUp, kRestUp))), p1, p2);
 }
 struct Pieces {
     uint32_t p0, p1, p2, h, l;
 };
-__device__ __forceinline__ Pieces split_field(float2 v) {
+__device__ __forceinline__ Pieces split_field(f32x2 v) {
     Pieces r;
     split_rest(v, r.p0, r.p1, r.p2);
     split_float(v, r.h, r.l);
@@ -110,11 +136,16 @@ struct FragShape {
     int tiles, steps;  // per block and per channel chunk
 };
 
-FragShape frag_shape(int cin, int cout) {
+// Two channel pairs a step (four would put the pieces of 4 more channels into registers: 760 bytes
+// spilled a thread, and an 8 -> 8 layer three times slower).  Row tiles up to the output channels, at most 4 (SU(2), SU(3)) or 2 (SU(4), whose
+// 4 tiles of sums, link and pieces spill 460 bytes: 18.8 ms against 15.6 ms for 4 layers of 8 channels
+// at 16^4, m = 8) and to the 227 KB of shared memory: more than that are further blocks, which load
+// the field again.
+FragShape frag_shape(int nc, int cin, int cout) {
     FragShape s;
     s.steps = cin <= 2 ? 1 : 2;
     s.ks = (cin + 2 * s.steps - 1) / (2 * s.steps) * s.steps;
-    s.tiles = cout <= 2 ? 1 : (cout <= 4 ? 2 : 4);
+    s.tiles = cout <= 2 ? 1 : (cout <= 4 || nc == 4 ? 2 : 4);
     if (s.tiles == 4 && (size_t)kPaths * 4 * s.ks * kStepBytes > 224 * 1024) s.tiles = 2;
     s.mt = (cout + 2 * s.tiles - 1) / (2 * s.tiles) * s.tiles;
     return s;
@@ -212,8 +243,8 @@ __global__ void ptc_prepare_kernel(PrepArgs a) {
                 v.x = scalbnf(v.x, e2) * sc;
                 v.y = scalbnf(v.y, e2) * sc;
             }
-            split_rest(make_float2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
-            split_rest(make_float2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
+            split_rest(pack2(v.x, -v.y), w0[2 * c], w1[2 * c], w2[2 * c]);               // real row
+            split_rest(pack2(v.y, v.x), w0[2 * c + 1], w1[2 * c + 1], w2[2 * c + 1]);   // imaginary row
         }
         uint4* f = L.frag + (int64_t)(((k * L.mt + mt) * L.ks + j)) * kStepVecs + lane;
         f[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
@@ -277,35 +308,6 @@ __device__ __forceinline__ void ptc_step(const Geom& g, const PtcSite& s, int k,
     link = (uint32_t)(2 * mu + (f ? s.p : 1 - s.p)) * vh + (f ? s.idx : nb);
 }
 
-// two FP32 numbers in one register pair and their packed arithmetic (same rounding as the
-// scalar instructions, half the issue slots)
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 __device__ __forceinline__ float2 cfma2(float2 a, float2 b, float2 c) {   // c + a b
     c.x = fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x));
     c.y = fmaf(a.x, b.y, fmaf(a.y, b.x, c.y));
@@ -320,7 +322,7 @@ __device__ __forceinline__ float2 cfma2(float2 a, float2 b, float2 c) {   // c +
 template <int NC, int MT, int KS>
 __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs a) {
     if (a.done != nullptr && *a.done) return;
-    constexpr int CG = NC == 4 && KS > 1 ? 2 : NC;
+    constexpr int CG = NC == 4 && KS > 1 ? 1 : NC;   // fewer spills than 2 or 4
     extern __shared__ uint4 sw[];
     const int mt0 = blockIdx.y * MT;
     const int per_path = MT * a.ks * kStepVecs;
@@ -390,8 +392,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
                 const float pc = chan[k * nch + 2 * j0 + i];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    x[i][c].x *= pc;
-                    x[i][c].y *= pc;
+                    x[i][c] = unpack2(mul2(pack2(x[i][c].x, x[i][c].y), pack2(pc, pc)));
                     mx = fmaxf(mx, fmaxf(fabsf(x[i][c].x), fabsf(x[i][c].y)));
                 }
             }
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs
                 for (int i = 0; i < 2 * KS; ++i)
 #pragma unroll
                     for (int c = 0; c < CG; ++c)
-                        y[i][c] = split_field(make_float2(x[i][c0 + c].x * sc, x[i][c0 + c].y * sc));
+                        y[i][c] = split_field(mul2(pack2(x[i][c0 + c].x, x[i][c0 + c].y), pack2(sc, sc)));
                 if (more) {
 #pragma unroll
                     for (int c = 0; c < CG; ++c) load_colour(next, j0, c0 + c);
@@ -532,14 +533,142 @@ int layer_launch(const LayerArgs& a, cudaStream_t st) {
 
 template <int NC>
 int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
+    if constexpr (NC < 4) {   // frag_shape
+        if (f.tiles == 4) return f.steps == 1 ? layer_launch<NC, 4, 1>(a, st) : layer_launch<NC, 4, 2>(a, st);
+    }
     switch (f.tiles * 2 + f.steps) {
         case 2 + 1: return layer_launch<NC, 1, 1>(a, st);
         case 2 + 2: return layer_launch<NC, 1, 2>(a, st);
         case 4 + 1: return layer_launch<NC, 2, 1>(a, st);
-        case 4 + 2: return layer_launch<NC, 2, 2>(a, st);
-        case 8 + 1: return layer_launch<NC, 4, 1>(a, st);
-        default: return layer_launch<NC, 4, 2>(a, st);
+        default: return layer_launch<NC, 2, 2>(a, st);
     }
+}
+
+// ---- layer in FP32 arithmetic ----
+// A thread per (site, output channel, RHS), which transports every input itself; the layer's
+// weights in shared memory.
+struct SimtArgs {
+    float2* out;
+    const float2* in;
+    const float2* w;
+    const float2* gauge;
+    Geom g;
+    int m, cin, cout, adj;
+    float t_sign;
+    const int* done;
+};
+constexpr int kSimtThreads = 256;
+
+// tv = U_k(x) f(x + k) for one RHS: f points at the channel's field + r
+template <int NC>
+__device__ __forceinline__ void ptc_transport(float2 (&tv)[4][NC], const float2* __restrict__ f,
+                                              const float2* __restrict__ U, int k, float sg, int m) {
+    if (k == 0) {
+#pragma unroll
+        for (int e = 0; e < 4 * NC; ++e) tv[e / NC][e % NC] = f[e * m];
+        return;
+    }
+    const bool fwd = (k & 1) != 0;
+    float2 u[NC][NC];
+#pragma unroll
+    for (int a = 0; a < NC; ++a)
+#pragma unroll
+        for (int b = 0; b < NC; ++b) {
+            const float2 e = fwd ? U[a * NC + b] : U[b * NC + a];
+            u[a][b] = make_float2(sg * e.x, fwd ? sg * e.y : -sg * e.y);
+        }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        float2 in[NC];
+#pragma unroll
+        for (int b = 0; b < NC; ++b) in[b] = f[(s * NC + b) * m];
+#pragma unroll
+        for (int a = 0; a < NC; ++a) {
+            float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int b = 0; b < NC; ++b) acc = cfma2(u[a][b], in[b], acc);
+            tv[s][a] = acc;
+        }
+    }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kSimtThreads, 2) ptc_simt_kernel(const SimtArgs a) {
+    if (a.done != nullptr && *a.done) return;
+    extern __shared__ float2 sw2[];   // [cout][cin][path][4][4]
+    const int cin = a.cin, cout = a.cout, m = a.m;
+    for (int e = threadIdx.x; e < cout * cin * kPaths * 16; e += blockDim.x) {
+        if (!a.adj) {
+            sw2[e] = a.w[e];
+        } else {   // W'[o][i][k][s'][s] = conj W[i][o][opposite k][s][s']
+            const int s = e & 3, sp = (e >> 2) & 3, k = (e >> 4) % kPaths, oi = (e >> 4) / kPaths;
+            const float2 v = a.w[(((int64_t)(oi % cin) * cout + oi / cin) * kPaths + opposite_path(k)) * 16 + s * 4 + sp];
+            sw2[e] = make_float2(v.x, -v.y);
+        }
+    }
+    __syncthreads();
+    const int per = m * cout, spb = blockDim.x / per;
+    if ((int)threadIdx.x >= spb * per) return;
+    const int r = threadIdx.x % m, o = (threadIdx.x / m) % cout;
+    const int64_t slen = 4 * NC * (int64_t)m, field = 2 * a.g.vh * slen;
+    for (int64_t site = (int64_t)blockIdx.x * spb + threadIdx.x / per; site < 2 * a.g.vh; site += (int64_t)gridDim.x * spb) {
+        const PtcSite ps = ptc_site(a.g, (uint32_t)site);
+        float2 acc[4][NC];
+#pragma unroll
+        for (int e = 0; e < 4 * NC; ++e) acc[e / NC][e % NC] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int k = 0; k < kPaths; ++k) {
+            uint32_t src = (uint32_t)site, link = 0;
+            bool wrap = false;
+            if (k) ptc_step(a.g, ps, k, src, link, wrap);
+#pragma unroll 1
+            for (int i = 0; i < cin; ++i) {
+                float2 tv[4][NC];
+                ptc_transport<NC>(tv, a.in + i * field + (int64_t)src * slen + r, a.gauge + (int64_t)link * (NC * NC), k,
+                                  wrap ? a.t_sign : 1.f, m);
+                const float2* W = sw2 + ((o * cin + i) * kPaths + k) * 16;
+#pragma unroll
+                for (int sp = 0; sp < 4; ++sp)
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        const float2 wv = W[sp * 4 + s];
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) acc[sp][c] = cfma2(wv, tv[s][c], acc[sp][c]);
+                    }
+            }
+        }
+        float2* dst = a.out + o * field + site * slen + r;
+#pragma unroll
+        for (int e = 0; e < 4 * NC; ++e) dst[e * m] = acc[e / NC][e % NC];
+    }
+}
+
+template <int NC>
+int simt_launch(const SimtArgs& a, cudaStream_t st) {
+    const size_t smem = (size_t)a.cout * a.cin * kPaths * 16 * sizeof(float2);
+    if (int rc = smem_optin(reinterpret_cast<const void*>(ptc_simt_kernel<NC>), smem)) return rc;
+    const int per = a.m * a.cout, block = kSimtThreads / per * per, spb = block / per;
+    const int64_t want = (2 * a.g.vh + spb - 1) / spb, cap = (int64_t)sm_count() * 8;
+    ptc_simt_kernel<NC><<<(int)(want < cap ? want : cap), block, smem, st>>>(a);
+    QCUB_CHECK_LAUNCH();
+    return QCU_SUCCESS;
+}
+
+// Whether FP32 arithmetic is the faster one.  Not for fewer columns than the MMA kernel takes in its
+// one wave of tiles: there it takes the time of one tile whatever the size (8^4, m = 1, the two edge
+// layers of an 8-channel network: 52 us against 84).  Above that the MMA's cost goes with the padded
+// channels, and one input or output channel fills half a K step or half a row tile while the link
+// works on every output channel.  16^4, SU(3), m = 8, us, FP32 arithmetic / MMA:
+//   1 -> 8 and 8 -> 1 together 1645 / 2320     2 -> 2 376 / 536     3 -> 3 851 / 900
+//   5 -> 5 (0.39 of the products of the padded tiles in use) 2330 / 2630, that of 6 -> 6 (0.56)
+// SU(4), and SU(2) where the field is loaded again for further row tiles, need 0.6 of the products in
+// use (SU(4), 6 -> 6, 0.56: 4520 / 5980 us; SU(2), 9 -> 9, 0.56: 4150 / 5460 us).  One or two right-hand
+// sides leave the FP32 kernel's rows short: with SU(2) and SU(3) only the edges are faster there.
+bool simt_faster(int nc, const FragShape& f, int cin, int cout, int m, int64_t vh) {
+    if (m * cout > kSimtThreads || 2 * vh * m <= (int64_t)sm_count() * (kMmaThreads / 32) * 8) return false;
+    if (cin == 1 || cout == 1 || cin * cout <= 4) return true;
+    const float need = nc == 4 || (nc == 2 && f.mt > f.tiles) ? 0.6f : 0.45f;
+    return (m >= 3 || nc == 4) && (cin * cout <= 9 || cin * cout < need * (4 * f.mt * f.ks));
 }
 
 // ---- weight gradient ----
@@ -694,7 +823,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
                 uint32_t p0[4], p1[4], p2[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    split_rest(make_float2(h[q][e][c].x * asc[e & 1], h[q][e][c].y * asc[e & 1]), p0[e], p1[e], p2[e]);
+                    split_rest(mul2(pack2(h[q][e][c].x, h[q][e][c].y), pack2(asc[e & 1], asc[e & 1])), p0[e], p1[e], p2[e]);
                 a0[q][c] = make_uint4(p0[0], p0[1], p0[2], p0[3]);
                 a1[q][c] = make_uint4(p1[0], p1[1], p1[2], p1[3]);
                 a2[q][c] = make_uint4(p2[0], p2[1], p2[2], p2[3]);
@@ -720,7 +849,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const float re = x[c][b].x * bsc, im = x[c][b].y * bsc;
-                    y[c][b] = split_field((g & 1) ? make_float2(-im, re) : make_float2(re, im));
+                    y[c][b] = split_field((g & 1) ? pack2(-im, re) : pack2(re, im));
                 }
 #pragma unroll
             for (int q = 0; q < MT; ++q) {
@@ -810,7 +939,6 @@ int grad_nc(const GradArgs& a, const GradShape& s, double2* gw, cudaStream_t st)
         case 16 + 4: return grad_launch<NC, 1, 4>(a, gw, s.nz, st);
         case 16 + 8: return grad_launch<NC, 1, 8>(a, gw, s.nz, st);
         case 32 + 1: return grad_launch<NC, 2, 1>(a, gw, s.nz, st);
-        case 32 + 4: return grad_launch<NC, 2, 4>(a, gw, s.nz, st);
         default: return grad_launch<NC, 2, 8>(a, gw, s.nz, st);
     }
 }
@@ -834,8 +962,8 @@ int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* 
     }
 }
 
-size_t ptc_frag_bytes(int cin, int cout) {
-    const FragShape f = frag_shape(cin, cout);
+size_t ptc_frag_bytes(int nc, int cin, int cout) {
+    const FragShape f = frag_shape(nc, cin, cout);
     const size_t b = (size_t)kPaths * (f.mt * f.ks * kStepBytes + (frag_channels(f.ks) + frag_rows(f.mt)) * sizeof(float));
     return (b + 15) & ~(size_t)15;
 }
@@ -855,13 +983,13 @@ FragParts frag_parts(void* base, const FragShape& f) {
 }
 }  // namespace
 
-int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
+int ptc_prepare(int nc, const float2* const* w, void* const* frag, const int* cin, const int* cout, int layers, bool adj,
                 cudaStream_t st) {
     PrepArgs a{};
     a.adj = adj;
     for (int l = 0; l < layers; ++l) {
         const int ci = adj ? cout[l] : cin[l], co = adj ? cin[l] : cout[l];
-        const FragShape f = frag_shape(ci, co);
+        const FragShape f = frag_shape(nc, ci, co);
         const FragParts p = frag_parts(frag[l], f);
         a.l[l] = PrepLayer{w[l], p.frag, p.chan, p.row, ci, co, f.mt, f.ks};
     }
@@ -870,9 +998,18 @@ int ptc_prepare(const float2* const* w, void* const* frag, const int* cin, const
     return QCU_SUCCESS;
 }
 
-int ptc_layer(int nc, float2* out, const float2* in, const void* frag, const float2* gauge, const Geom& g, int m,
-              int cin, int cout, float t_sign, const int* done, cudaStream_t st) {
-    const FragShape f = frag_shape(cin, cout);
+int ptc_layer(int nc, float2* out, const float2* in, const float2* w, bool adj, const void* frag, const float2* gauge,
+              const Geom& g, int m, int cin, int cout, float t_sign, const int* done, cudaStream_t st) {
+    const FragShape f = frag_shape(nc, cin, cout);
+    if (simt_faster(nc, f, cin, cout, m, g.vh)) {
+        const SimtArgs a{out, in, w, gauge, g, m, cin, cout, adj, t_sign, done};
+        switch (nc) {
+            case 2: return simt_launch<2>(a, st);
+            case 3: return simt_launch<3>(a, st);
+            case 4: return simt_launch<4>(a, st);
+            default: return set_error(QCU_ERR_UNSUPPORTED, "preconditioner n_color=%d (2..4)", nc);
+        }
+    }
     const FragParts p = frag_parts(const_cast<void*>(frag), f);
     const LayerArgs a{out, in, p.frag, p.chan, p.row, gauge, g, m, cin, cout, f.mt, f.ks, t_sign, done};
     switch (nc) {

@@ -192,6 +192,26 @@ def test_apply_keeps_the_range_of_fp32(oracle_lib, L, nc, m, layers, ch, size):
     assert rel_err(_apply(L, nc, m, layers, ch, g, ws, b), ref) <= 2e-6
 
 
+# more columns than one wave of the MMA kernel's tiles: FP32 arithmetic in the layers that it suits
+# (one channel on a side, few channels, SU(2) and SU(4) with 6), the MMA in the others and where a
+# block would not hold m channels threads
+LARGE = [((8, 8, 4, 6), 3, 7, 3, 2), ((8, 6, 6, 6), 2, 6, 3, 6), ((6, 8, 6, 6), 4, 6, 3, 6), ((8, 8, 8, 4), 3, 5, 3, 5),
+         ((8, 4, 6, 8), 3, 9, 3, 3), ((4, 4, 4, 4), 3, 64, 2, 8), ((6, 6, 6, 8), 4, 6, 1, 1)]
+
+
+@pytest.mark.parametrize("L,nc,m,layers,ch", LARGE)
+def test_layers_of_large_lattices(oracle_lib, L, nc, m, layers, ch):
+    kappa = 0.12
+    g, ws, b = _case(L, nc, m, layers, ch, 1100 + ch + m, 1.0)
+    ref = oracle_lib.precond_apply(b, ws, g, L, -1.0)
+    assert rel_err(_apply(L, nc, m, layers, ch, g, ws, b), ref) <= 2e-6
+    loss, grads = _loss_grad(L, nc, m, layers, ch, g, ws, b, kappa)
+    ref_loss, ref_grads = oracle_lib.precond_loss_grad(b, ws, g, L, kappa, -1.0)
+    assert loss == pytest.approx(ref_loss, rel=4e-6)
+    for gg, rg in zip(grads, ref_grads):
+        assert rel_err(gg, rg) <= 4e-6
+
+
 def test_gradient_beside_an_infinite_channel(oracle_lib):
     """A channel whose output gradient overflows (its last weight is near FP32's largest number, its
     own value is zero) leaves the other channels' gradients as they are."""
