@@ -209,8 +209,9 @@ __device__ __forceinline__ void hop_site(typename St<S>::A2 (&acc)[4][NC], const
 // Epilogue of one (site, RHS): store out = D in (EPI_PLAIN) or the fused combination
 // with x / r0, and add this thread's terms of the fused reductions to red.
 // `base` is the offset of (site, spin 0, colour 0, RHS) in the gathered layout; row i of x
-// (r0) is at xv[i xs] (r0[i rs]), in global or shared memory.
-template <int NC, typename S, int EPI, int NV>
+// (r0) is at xv[i xs] (r0[i rs0]), in global or shared memory, or (INDEXED) at its place in the
+// vector x.
+template <int NC, typename S, int EPI, int NV, bool INDEXED = false>
 __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC], const HopParams& p,
                                           int64_t base, typename St<S>::A2 (&red)[NV > 0 ? NV : 1],
                                           const typename St<S>::S2* __restrict__ xv, int xs,
@@ -230,7 +231,7 @@ __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC]
             if (EPI == EPI_PLAIN) {
                 out[o] = St<S>::cv(v);
             } else {
-                const A2 xx = St<S>::ld(xv[(s * NC + c) * xs]);
+                const A2 xx = St<S>::ld(xv[INDEXED ? o : (s * NC + c) * xs]);
                 const A a = (A)p.a;
                 A2 res;
                 if (EPI == EPI_XPAY) {
@@ -263,13 +264,16 @@ __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC]
         }
 }
 
-// the same with x and r0 read from their vectors
+// The same with x and r0 read from their vectors.  x of the x + a D in form by its place in the vector
+// up to N = 6, else from a moved base: FP64, 16^4, m = 12, us, 330 / 382 at N = 5, 433 / 477 at N = 6 and
+// 708 / 653 at N = 7 (the compiler schedules the two differently).
 template <int NC, typename S, int EPI, int NV>
 __device__ __forceinline__ void hop_store(const typename St<S>::A2 (&acc)[4][NC], const HopParams& p,
                                           int64_t base, typename St<S>::A2 (&red)[NV > 0 ? NV : 1]) {
     using S2 = typename St<S>::S2;
-    hop_store<NC, S, EPI, NV>(acc, p, base, red, static_cast<const S2*>(p.x) + base, p.m,
-                              static_cast<const S2*>(p.r0) + base, p.m);
+    constexpr bool INDEXED = EPI == EPI_XPAY && NC <= 6;
+    hop_store<NC, S, EPI, NV, INDEXED>(acc, p, base, red, static_cast<const S2*>(p.x) + (INDEXED ? 0 : base), p.m,
+                                       static_cast<const S2*>(p.r0) + base, p.m);
 }
 
 // Minimum resident blocks per SM requested from the register allocator: FP64 at small N
@@ -288,13 +292,16 @@ struct HopMinBlocks {
 //   16^4, N = 6, m = 8       FP32 169 -> 103, 165 -> 120
 // The limit leaves L1 room for the links, which all RHS of a site read: with x and r0 both
 // staged in FP64 at N = 3 (192 KB) the <r0, v> form took 1721 us.
+// Not staged, since it was slower than reading after the hop (mean over 8^4, 16^4 and m = 1..32):
+// r0 of 16-bit storage at N = 4 (1.03, 1.13 at m = 5; x alone 0.96), and x of the residual form where
+// r0 does not fit beside it (FP32 1.05 at N = 6, 1.02 at N = 4; FP64 the same with and without).
 template <int NC, typename S, int EPI>
 struct HopStage {
     static constexpr int kReads = EPI == EPI_PLAIN ? 0 : ((EPI == EPI_SCHUR_R0 || EPI == EPI_RESID) ? 2 : 1);
     static constexpr int kVecBytes = 4 * NC * kRedThreads * 2 * (int)sizeof(S);   // one vector, one block
     static constexpr int kBlocks = HopMinBlocks<NC, S>::value < 2 ? 2 : HopMinBlocks<NC, S>::value;
-    static constexpr int kFit = 150 * 1024 / (kVecBytes * kBlocks);
-    static constexpr int value = kReads < kFit ? kReads : kFit;
+    static constexpr int kFit = NC == 4 && sizeof(S) == 2 ? 1 : 150 * 1024 / (kVecBytes * kBlocks);
+    static constexpr int value = kReads <= kFit ? kReads : (EPI == EPI_RESID ? 0 : kFit);
 };
 
 // asynchronous 4-, 8- or 16-byte copy of one complex number into shared memory

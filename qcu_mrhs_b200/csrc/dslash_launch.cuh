@@ -40,7 +40,8 @@ int launch_hop(const HopParams& p, bool dagger, int epi, cudaStream_t stream, bo
     if (!color_split) {
         switch (epi) {
             case EPI_PLAIN: break;
-            case EPI_SCHUR_R0: case EPI_RESID: smem = HopStage<NC, S, EPI_RESID>::value; break;
+            case EPI_SCHUR_R0: smem = HopStage<NC, S, EPI_SCHUR_R0>::value; break;
+            case EPI_RESID: smem = HopStage<NC, S, EPI_RESID>::value; break;
             default: smem = HopStage<NC, S, EPI_XPAY>::value;
         }
         smem *= (size_t)4 * NC * block * 2 * sizeof(S);
