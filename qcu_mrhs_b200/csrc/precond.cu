@@ -216,9 +216,8 @@ int Precond::init(const int L[4], int n_color, int m_rhs, int n_layers, int chan
     if (n_layers < 1 || n_layers > 16) return set_error(QCU_ERR_INVALID, "layers=%d (1..16)", n_layers);
     if (channels < 1 || channels > 16 || (n_layers == 1 && channels != 1))
         return set_error(QCU_ERR_INVALID, "channels=%d (1..16; 1 for a single layer)", channels);
-    if (m_rhs * channels > 1024) return set_error(QCU_ERR_UNSUPPORTED, "m_rhs * channels > 1024");
-    if ((size_t)channels * channels * kPaths * 16 * sizeof(float2) > 200 * 1024)
-        return set_error(QCU_ERR_UNSUPPORTED, "channels=%d: one layer's weights exceed shared memory", channels);
+    // a layer's weights in FP32 (180 KB at 13) in the shared memory of ptc_simt_kernel
+    if (channels > 13) return set_error(QCU_ERR_UNSUPPORTED, "channels=%d (at most 13)", channels);
     if (t_boundary != 1.0 && t_boundary != -1.0) return set_error(QCU_ERR_INVALID, "t_boundary must be +1 or -1");
     g = make_geom(L);
     nc = n_color;

@@ -1,12 +1,12 @@
-"""The tensor-core layer and weight-gradient kernels of the learned preconditioner at the
-edges of their tiles: columns (site, RHS) in tiles of 8 (odd m: two sites in a lane's column
-pair; a last tile that is not full), output channels in tiles of 2 and 4, input channels in
-steps of 2 and chunks of 4 or 8, against the oracle.
+"""The layer and weight-gradient kernels of the learned preconditioner at the edges of their
+tiles: columns (site, RHS) in tiles of 8 (odd m: two sites in a lane's column pair; a last tile
+that is not full), output channels in tiles of 2 and 4, input channels in steps of 2 and 4 and
+chunks of 4 or 8, against the oracle; and with right-hand sides, channels, spins and single weights
+of very different size, for which FP32 arithmetic needs no special case.
 
-Tolerances: the kernels' products are exact to 2^-20 with errors of random sign, and a
-network of `layers` layers sums at most 13 x 9 x 4 of them per output, so 2e-6 holds the
-output of 2-3 layers and 4e-6 the gradient (which also carries the adjoint layers) with a
-margin of about 4 over the errors of 2^-20 sqrt(layers)."""
+Tolerances: an output is a chain of at most 16 N + 1 = 65 FP32 additions per 4 input channels, so
+its error is about 2^-24 sqrt(65) = 4.8e-7 of it a layer and 8.3e-7 after three layers: 2e-6 for
+the output.  The gradient follows the layers and their adjoints, 1.2e-6: 4e-6."""
 import numpy as np
 import pytest
 
