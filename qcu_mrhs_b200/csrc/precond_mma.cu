@@ -34,6 +34,8 @@
 // 8..15 the imaginary parts: a lane's D registers are whole complex numbers.
 //
 // No reference code; the CPU restatement oracle_ptc_forward is the checker.
+#include <utility>
+
 #include "precond.h"
 
 namespace qcub {
@@ -654,27 +656,34 @@ int simt_launch(const SimtArgs& a, cudaStream_t st) {
     return QCU_SUCCESS;
 }
 
-// Whether FP32 arithmetic is the faster one.  Not for fewer columns than the MMA kernel takes in its
-// one wave of tiles: there it takes the time of one tile whatever the size (8^4, m = 1, the two edge
-// layers of an 8-channel network: 52 us against 84).  Above that the MMA's cost goes with the padded
-// channels, and one input or output channel fills half a K step or half a row tile while the link
-// works on every output channel.  16^4, SU(3), m = 8, us, FP32 arithmetic / MMA:
+// Whether FP32 arithmetic is the faster one.
+// One input channel: at every size (2^4 to 8^4, SU(3), m = 3, 1 -> 8: 15-37 us against 27-48), but for
+// SU(4) with a short row on a small lattice (4^4, m = 1, 1 -> 1: 45 / 22 us; m cout = 4: 22 / 26).
+// More: not for fewer columns than the MMA kernel takes in its one wave of tiles, where it takes the
+// time of one tile whatever the size (8^4, m = 1, 8 -> 1: 68 / 36 us).  Above that the MMA's cost goes
+// with the padded channels, and one output channel fills half a row tile.  16^4, SU(3), m = 8:
 //   1 -> 8 and 8 -> 1 together 1645 / 2320     2 -> 2 376 / 536     3 -> 3 851 / 900
 //   5 -> 5 (0.39 of the products of the padded tiles in use) 2330 / 2630, that of 6 -> 6 (0.56)
 // SU(4), and SU(2) where the field is loaded again for further row tiles, need 0.6 of the products in
 // use (SU(4), 6 -> 6, 0.56: 4520 / 5980 us; SU(2), 9 -> 9, 0.56: 4150 / 5460 us).  One or two right-hand
 // sides leave the FP32 kernel's rows short: with SU(2) and SU(3) only the edges are faster there.
 bool simt_faster(int nc, const FragShape& f, int cin, int cout, int m, int64_t vh) {
-    if (m * cout > kSimtThreads || 2 * vh * m <= (int64_t)sm_count() * (kMmaThreads / 32) * 8) return false;
-    if (cin == 1 || cout == 1 || cin * cout <= 4) return true;
+    if (m * cout > kSimtThreads) return false;
+    const bool large = 2 * vh * m > (int64_t)sm_count() * (kMmaThreads / 32) * 8;
+    if (cin == 1) return nc < 4 || large || m * cout >= 4;
+    if (!large) return false;
+    if (cout == 1 || cin * cout <= 4) return true;
     const float need = nc == 4 || (nc == 2 && f.mt > f.tiles) ? 0.6f : 0.45f;
     return (m >= 3 || nc == 4) && (cin * cout <= 9 || cin * cout < need * (4 * f.mt * f.ks));
 }
 
 // ---- weight gradient ----
 // gw[o][i][k][s'][s] = sum_{x, c, r} g_o[s'][c][r](x) conj((T_k in_i)[s][c][r](x))
-//                    = sum_{x, c, r} (U_k^dag g_o)[s'][c][r](x) conj(in_i[s][c][r](x + k)):
-// one matrix product per path over all columns.  A: rows (o, s'), K = (column, re/im) of the
+//                    = sum_{x, c, r} (U_k^dag g_o)[s'][c][r](x) conj(in_i[s][c][r](x + k))
+//                    = conj sum_{x, c, r} (U_-k^dag in_i)[s][c][r](x) conj(g_o[s'][c][r](x - k)):
+// one matrix product per path over all columns, of the first form or, for one output channel of
+// several inputs (4 of 16 rows in the first form), of the last: the same sum with the two fields'
+// parts exchanged, path -k for k.  In the first form's terms, A: rows (o, s'), K = (column, re/im) of the
 // transported gradient; B: columns (i, s, re/im), the pair (v.re, v.im) for the real part and
 // (-v.im, v.re) for the imaginary part, so a lane's D registers are whole complex numbers.
 // A column is a (site, RHS) pair, and the operands' sizes run in opposite directions: the loss
@@ -697,6 +706,7 @@ struct GradArgs {
     const double* bnorm;   // ||b_j||
     Geom g;
     int m, cin, cout;
+    bool swapped;          // gout is the layer's input, in its output gradient
     float t_sign;
 };
 
@@ -719,7 +729,7 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
     if (threadIdx.x < a.m) {
         float inv;
         const float p = power_of((float)a.bnorm[threadIdx.x], &inv);
-        sizes[threadIdx.x] = make_float2(p, inv);
+        sizes[threadIdx.x] = a.swapped ? make_float2(inv, p) : make_float2(p, inv);
     }
     __syncthreads();
     constexpr int NA = MT * CI * 4;
@@ -885,9 +895,10 @@ __global__ void __launch_bounds__(kGradWarps * 32, 1) ptc_grad_kernel(const Grad
     }
 }
 
-// sum of the chunks, into gw
-__global__ void ptc_grad_sum_kernel(double2* __restrict__ gw, const double* __restrict__ part, int chunks, int mt, int ci,
-                                    int cin, int cout, int nz) {
+// sum of the chunks, into gw; swapped: of the exchanged form, element (o, i, k, s', s) to the conjugate
+// at (i, o, -k, s, s')
+__global__ void ptc_grad_sum_kernel(double2* __restrict__ gw, const double* __restrict__ part, int mt, int ci,
+                                    int cin, int cout, int nz, bool swapped) {
     const int na = mt * ci * 128;   // doubles of one (chunk, path, z)
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= kPaths * nz * na / 2) return;
@@ -901,13 +912,21 @@ __global__ void ptc_grad_sum_kernel(double2* __restrict__ gw, const double* __re
     if (ii >= cin || o >= cout) return;
     const double* src = part + ((size_t)k * nz + z) * na + ((tile * ci + i) * 4 + 2 * w) * 32 + lane;
     double2 s = make_double2(0.0, 0.0);
-    for (int c = 0; c < chunks; ++c) {
+#pragma unroll
+    for (int c = 0; c < kGradChunks; ++c) {
         s.x += src[(size_t)c * kPaths * nz * na];
         s.y += src[(size_t)c * kPaths * nz * na + 32];
     }
-    gw[(((int64_t)o * cin + ii) * kPaths + k) * 16 + ((lane >> 2) & 3) * 4 + (lane & 3)] = s;
+    const int sp = (lane >> 2) & 3, sc = lane & 3;
+    if (swapped)
+        gw[(((int64_t)ii * cout + o) * kPaths + opposite_path(k)) * 16 + sc * 4 + sp] = make_double2(s.x, -s.y);
+    else
+        gw[(((int64_t)o * cin + ii) * kPaths + k) * 16 + sp * 4 + sc] = s;
 }
 
+bool grad_swapped(int cin, int cout) { return cout == 1 && cin > 1; }
+
+// Row tiles of 4 output channels and input channels of a block: all of up to 8 x 8.
 struct GradShape {
     int mt, ci, nz;
 };
@@ -927,7 +946,7 @@ int grad_launch(const GradArgs& a, double2* gw, int nz, cudaStream_t st) {
     k<<<dim3(kGradChunks, kPaths, (unsigned)nz), kGradWarps * 32, smem, st>>>(a);
     QCUB_CHECK_LAUNCH();
     const int n = kPaths * nz * MT * CI * 64;
-    ptc_grad_sum_kernel<<<(n + 255) / 256, 256, 0, st>>>(gw, a.part, kGradChunks, MT, CI, a.cin, a.cout, nz);
+    ptc_grad_sum_kernel<<<(n + 255) / 256, 256, 0, st>>>(gw, a.part, MT, CI, a.cin, a.cout, nz, a.swapped);
     QCUB_CHECK_LAUNCH();
     return QCU_SUCCESS;
 }
@@ -937,7 +956,6 @@ int grad_nc(const GradArgs& a, const GradShape& s, double2* gw, cudaStream_t st)
     switch (s.mt * 16 + s.ci) {
         case 16 + 1: return grad_launch<NC, 1, 1>(a, gw, s.nz, st);
         case 16 + 4: return grad_launch<NC, 1, 4>(a, gw, s.nz, st);
-        case 16 + 8: return grad_launch<NC, 1, 8>(a, gw, s.nz, st);
         case 32 + 1: return grad_launch<NC, 2, 1>(a, gw, s.nz, st);
         default: return grad_launch<NC, 2, 8>(a, gw, s.nz, st);
     }
@@ -946,14 +964,18 @@ int grad_nc(const GradArgs& a, const GradShape& s, double2* gw, cudaStream_t st)
 }  // namespace
 
 size_t ptc_grad_bytes(int cin, int cout) {
-    const GradShape s = grad_shape(cin, cout);
+    const GradShape s = grad_shape(grad_swapped(cin, cout) ? cout : cin, grad_swapped(cin, cout) ? cin : cout);
     return (size_t)kGradChunks * kPaths * s.nz * s.mt * s.ci * 128 * sizeof(double);
 }
 
 int ptc_grad(int nc, double2* gw, void* part, const float2* gout, const float2* in, const float2* gauge,
              const double* bnorm, const Geom& g, int m, int cin, int cout, float t_sign, cudaStream_t st) {
-    const GradShape s = grad_shape(cin, cout);
-    const GradArgs a{static_cast<double*>(part), gout, in, gauge, bnorm, g, m, cin, cout, t_sign};
+    GradArgs a{static_cast<double*>(part), gout, in, gauge, bnorm, g, m, cin, cout, grad_swapped(cin, cout), t_sign};
+    if (a.swapped) {
+        std::swap(a.gout, a.in);
+        std::swap(a.cin, a.cout);
+    }
+    const GradShape s = grad_shape(a.cin, a.cout);
     switch (nc) {
         case 2: return grad_nc<2>(a, s, gw, st);
         case 3: return grad_nc<3>(a, s, gw, st);
