@@ -664,17 +664,21 @@ int simt_launch(const SimtArgs& a, cudaStream_t st) {
 // with the padded channels, and one output channel fills half a row tile.  16^4, SU(3), m = 8:
 //   1 -> 8 and 8 -> 1 together 1645 / 2320     2 -> 2 376 / 536     3 -> 3 851 / 900
 //   5 -> 5 (0.39 of the products of the padded tiles in use) 2330 / 2630, that of 6 -> 6 (0.56)
-// SU(4), and SU(2) where the field is loaded again for further row tiles, need 0.6 of the products in
+// SU(4), and SU(2) where the field is loaded again for further row tiles, need more of the products in
 // use (SU(4), 6 -> 6, 0.56: 4520 / 5980 us; SU(2), 9 -> 9, 0.56: 4150 / 5460 us).  One or two right-hand
-// sides leave the FP32 kernel's rows short: with SU(2) and SU(3) only the edges are faster there.
+// sides leave the FP32 kernel's rows short: with SU(2) and SU(3) only the edges are faster there.  A last
+// wave that is mostly empty counts as padding (8^4, SU(3), m = 3, 6 -> 6: 80 / 120 us).
 bool simt_faster(int nc, const FragShape& f, int cin, int cout, int m, int64_t vh) {
     if (m * cout > kSimtThreads) return false;
-    const bool large = 2 * vh * m > (int64_t)sm_count() * (kMmaThreads / 32) * 8;
+    const int64_t cols = 2 * vh * m, tiles = (kMmaThreads / 32) * 8;   // of one block
+    const bool large = cols > sm_count() * tiles;
     if (cin == 1) return nc < 4 || large || m * cout >= 4;
     if (!large) return false;
     if (cout == 1 || cin * cout <= 4) return true;
-    const float need = nc == 4 || (nc == 2 && f.mt > f.tiles) ? 0.6f : 0.45f;
-    return (m >= 3 || nc == 4) && (cin * cout <= 9 || cin * cout < need * (4 * f.mt * f.ks));
+    const float need = nc == 4 ? 0.6f : (nc == 2 && f.mt > f.tiles ? 0.57f : 0.45f);
+    const int64_t wave = max(sm_count() * f.tiles / f.mt, 1) * tiles;
+    const float filled = (float)cols / (float)((cols + wave - 1) / wave * wave);
+    return (m >= 3 || nc == 4) && (cin * cout <= 9 || cin * cout * filled < need * (4 * f.mt * f.ks));
 }
 
 // ---- weight gradient ----
