@@ -1,4 +1,5 @@
-// precond_mma.cu -- tensor-core kernels of the learned preconditioner (precond.h).
+// precond_mma.cu -- layers and weight gradient of the learned preconditioner (precond.h), on the
+// tensor cores and, for layers that would mostly pad their tiles, in FP32 arithmetic.
 //
 // Layer: out_o(x) = sum_k U_k(x) [ sum_i W[o][i][k] in_i(x + k) ], k = 0..8, with U_0 = 1.
 // The spin mixing in brackets is one matrix product per path, the same weights for every
@@ -12,7 +13,7 @@
 // linear network is free to shift factors, nor that of a right-hand side costs bits.
 //   first pieces  w0, x0: the values rounded to multiples of 2^6, so 9 bits of the largest entry.
 //                 Products of two of them are multiples of 2^12 up to 2^30, and 64 of them (the
-//                 largest K that one accumulator sees) add up within 24 bits: exact.
+//                 gradient's K; a layer's is 32) add up within 24 bits: exact.
 //   the rest      w x = w0 x0 + w0 (x - x0) + (w - w0) x, with x - x0 = (x1 + x2) / 2^9,
 //                 w - w0 = (w1 + w2) / 2^9 and x = h + l: w0 x1 + w0 x2 + w1 h + w1 l + w2 h, five
 //                 more products.  The factor 2^9 keeps the pieces clear of FP16's subnormal
@@ -320,7 +321,10 @@ __device__ __forceinline__ float2 cfma2(float2 a, float2 b, float2 c) {   // c +
 // colours, 2 MT output channels, input channels 2 KS at a time.  The block's weights (its MT row
 // tiles) stay in shared memory (216 KB for 8 x 8 channels), so one block of 8 warps runs on an SM, at
 // up to 255 registers: a step's spinors and link are requested under the products of the step
-// before it.
+// before it.  16^4, SU(3), m = 8, one 8 -> 8 layer: 6.5 ms as FP32 arithmetic with a thread per (site,
+// output channel, RHS); 1.86 ms with five products, two pieces of a field and one scale for many
+// channels, which lost bits of all but the largest entries; 2.64 ms so.  6 MT KS NC MMAs a step (288 a
+// path) bound it at 1.26 ms; the rest is the fixed latency of the MMA and FP32 chains at 8 warps.
 template <int NC, int MT, int KS>
 __global__ void __launch_bounds__(kMmaThreads, 1) ptc_mma_kernel(const LayerArgs a) {
     if (a.done != nullptr && *a.done) return;
@@ -548,7 +552,7 @@ int layer_nc(const LayerArgs& a, const FragShape& f, cudaStream_t st) {
 
 // ---- layer in FP32 arithmetic ----
 // A thread per (site, output channel, RHS), which transports every input itself; the layer's
-// weights in shared memory.
+// weights in shared memory.  FP32 issue bounds it (62 % at 24 % of the warps).
 struct SimtArgs {
     float2* out;
     const float2* in;
@@ -699,6 +703,9 @@ bool simt_faster(int nc, const FragShape& f, int cin, int cout, int m, int64_t v
 // Both operands keep 24 bits as the layer's: the first pieces' products add up exactly (K <= 64), the
 // other five go to a second accumulator.  A step's products (6 NC MMAs per tile, one rounding)
 // are added to FP64 sums in shared memory; warps, blocks and chunks are summed in a fixed order.
+// 8^3x16, SU(3), m = 8, 8 -> 8 and 8 -> 1: 1358 and 693 us as FP32 arithmetic with a block per (o, i, k),
+// 449 and 295 us with four products, shared scales and FP32 sums of 8 steps, 625 and 221 us so (the
+// second with the fields exchanged; 442 us without).  MMA and FP32 chain latency at 8 warps bound it.
 constexpr int kGradWarps = 8;
 constexpr int kGradChunks = 16;   // blocks per path: 9 x 16 blocks of 8 warps, one per SM
 
